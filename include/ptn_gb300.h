@@ -71,6 +71,17 @@ typedef struct {
  * and contract_nodes (contractions/node_contraction.py:62-86). */
 int ptn_zcontract(const ptn_contract_desc* d, void* stream);
 
+/* The same contraction with device scratch: contractions with enough
+ * arithmetic run as exact integer digit products on the tensor cores (operands
+ * rounded at 2^-56 of each row's largest entry, sums exact, one rounding to
+ * double), whose error is not above the FP64 kernels'; the others, and calls
+ * with null, misaligned (256 bytes) or too little scratch, run as
+ * ptn_zcontract. ptn_zcontract_work_bytes: the scratch the call needs, 0 when
+ * the FP64 kernels take it (host arithmetic on the descriptor's sizes). The
+ * result does not vary between runs. Same counterparts as ptn_zcontract. */
+int64_t ptn_zcontract_work_bytes(const ptn_contract_desc* d);
+int ptn_zcontract_ws(const ptn_contract_desc* d, void* work, int64_t work_bytes, void* stream);
+
 /* The K split ptn_zcontract uses for an output of `tiles` 64 x 64 tiles and a
  * K range of K: returns the number of splits and sets *k_chunk (K indices per
  * split). Host-only arithmetic. No counterpart in the reference. */
@@ -316,11 +327,12 @@ int ptn_zpermute(const ptn_permute_desc* d, void* stream);
  * run with different vectors. Replaces the Python loop over np.tensordot calls
  * of contract_ket_ham_with_envs / contract_any
  * (contractions/state_operator_contraction.py:227-273, 407-694) with one call. */
-enum { PTN_OP_ZCONTRACT = 0, PTN_OP_CGEMM = 1, PTN_OP_TO_PLANES = 2, PTN_OP_EXPAND_B = 3 };
+enum { PTN_OP_ZCONTRACT = 0, PTN_OP_CGEMM = 1, PTN_OP_TO_PLANES = 2, PTN_OP_EXPAND_B = 3, PTN_OP_ZCONTRACT_WS = 4 };
 typedef struct {
   int32_t kind;
   int32_t a, b, c;
-  int32_t d;                /* PTN_OP_CGEMM: table index of the split-K scratch, or -1 */
+  int32_t d;                /* PTN_OP_CGEMM: table index of the split-K scratch, or -1;
+                               PTN_OP_ZCONTRACT_WS: of ptn_zcontract_work_bytes(desc) bytes, or -1 */
   int32_t pad_;
   const void* desc;
 } ptn_exec_op;

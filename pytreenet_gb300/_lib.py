@@ -88,13 +88,15 @@ class ExecOp(ctypes.Structure):
                 ("desc", ctypes.c_void_p)]
 
 
-OP_ZCONTRACT, OP_CGEMM, OP_TO_PLANES, OP_EXPAND_B = 0, 1, 2, 3
+OP_ZCONTRACT, OP_CGEMM, OP_TO_PLANES, OP_EXPAND_B, OP_ZCONTRACT_WS = 0, 1, 2, 3, 4
 
 _P = ctypes.c_void_p
 _I64 = ctypes.c_int64
 _I32 = ctypes.c_int32
 SIGNATURES = {
     "ptn_zcontract": (ctypes.c_int, [ctypes.POINTER(ContractDesc), _P]),
+    "ptn_zcontract_work_bytes": (_I64, [ctypes.POINTER(ContractDesc)]),
+    "ptn_zcontract_ws": (ctypes.c_int, [ctypes.POINTER(ContractDesc), _P, _I64, _P]),
     "ptn_zcontract_splits": (_I64, [_I64, _I64, ctypes.POINTER(ctypes.c_int64)]),
     "ptn_krylov_partials": (_I64, [_I64]),
     "ptn_zdot_multi": (ctypes.c_int, [_P, _I64, _I32, _P, _I64, _P, _I32, _P, _P]),

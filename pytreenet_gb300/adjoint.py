@@ -127,14 +127,17 @@ def _raw_contract(a, la, b, lb, lc, klabels, conj_a=False, conj_b=False, out=Non
         st = Step(Operand.contiguous(("fixed", None), la, list(a.shape)),
                   Operand.contiguous(("fixed", None), lb, list(b.shape)), list(klabels),
                   Operand.contiguous(("fixed", None), lc, shape_c), conj_a=conj_a, conj_b=conj_b, beta=beta)
+        wb = E.contract_work_bytes(st.desc, a.device)
         ops = (_lib.ExecOp * 1)()
-        ops[0].kind = _lib.OP_ZCONTRACT
-        ops[0].a, ops[0].b, ops[0].c = 2, 3, 4
+        ops[0].kind = _lib.OP_ZCONTRACT_WS if wb else _lib.OP_ZCONTRACT
+        ops[0].a, ops[0].b, ops[0].c, ops[0].d = 2, 3, 4, 1 if wb else -1
         ops[0].desc = ctypes.addressof(st.desc)
-        ent = (st, ops)
+        ent = (st, ops, wb)
         _DESCS[key] = ent
-    st, ops = ent
-    ptrs = (ctypes.c_void_p * 5)(None, None, a.data_ptr(), b.data_ptr(), out.data_ptr())
+    st, ops, wb = ent
+    # scratch per call: contractions of several threads and streams may overlap
+    work = torch.empty(wb, dtype=torch.uint8, device=a.device) if wb else None
+    ptrs = (ctypes.c_void_p * 5)(None, work.data_ptr() if wb else None, a.data_ptr(), b.data_ptr(), out.data_ptr())
     check(_lib.load().ptn_exec_ops(ops, 1, ptrs, 5, E._stream_ptr()), "ptn_exec_ops")
     return out
 

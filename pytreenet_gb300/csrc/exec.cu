@@ -27,6 +27,15 @@ extern "C" int ptn_exec_ops(const ptn_exec_op* ops, int32_t nops, void* const* p
         st = ptn_zcontract(&d, stream);
         break;
       }
+      case PTN_OP_ZCONTRACT_WS: {
+        ptn_contract_desc d = *static_cast<const ptn_contract_desc*>(op.desc);
+        d.A = ptrs[op.a];
+        d.B = op.b >= 0 ? ptrs[op.b] : nullptr;
+        d.C = ptrs[op.c];
+        void* work = op.d >= 0 ? ptrs[op.d] : nullptr;
+        st = ptn_zcontract_ws(&d, work, work ? ptn_zcontract_work_bytes(&d) : 0, stream);
+        break;
+      }
       case PTN_OP_CGEMM: {
         ptn_cgemm_desc d = *static_cast<const ptn_cgemm_desc*>(op.desc);
         d.A = ptrs[op.a];

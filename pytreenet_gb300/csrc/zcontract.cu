@@ -18,44 +18,11 @@
 // adds alpha times its partial sums with double-precision atomics. The
 // summation order then varies between runs at the level of rounding.
 #include "ptn_common.cuh"
+#include "zmodes.cuh"
 
 namespace {
 
 constexpr int BM = 64, BN = 64, BK = 8;
-
-struct ModeDev {
-  int n;
-  int64_t dim[PTN_MAX_MODES];
-  int64_t s0[PTN_MAX_MODES];
-  int64_t s1[PTN_MAX_MODES];
-};
-
-struct ContractArgs {
-  const double2* A;
-  const double2* B;
-  double2* C;
-  double2 alpha, beta;
-  int conj_a, conj_b;
-  int beta_zero;
-  int64_t M, N, K;
-  int64_t tiles_n;
-  int64_t k_chunk;  // K indices per split (the whole K when not split)
-  int split;        // accumulate with atomics into a pre-scaled C
-  ModeDev m, n, k;  // m: (A, C) strides; n: (B, C); k: (A, B)
-};
-
-__device__ __forceinline__ void decode(const ModeDev& md, int64_t idx, int64_t& o0, int64_t& o1) {
-  o0 = 0;
-  o1 = 0;
-  for (int d = md.n - 1; d >= 0; --d) {
-    int64_t dd = md.dim[d];
-    int64_t q = idx / dd;
-    int64_t r = idx - q * dd;
-    o0 += r * md.s0[d];
-    o1 += r * md.s1[d];
-    idx = q;
-  }
-}
 
 __global__ void __launch_bounds__(256) zcontract_kernel(const ContractArgs a) {
   __shared__ double2 As[BK][BM];
@@ -307,7 +274,7 @@ __global__ void __launch_bounds__(ELEM_THREADS) zcontract_elem_kernel(const Cont
   }
 }
 
-// C <- beta * C (zero when beta == 0) over the M x N output positions.// C <- beta * C (zero when beta == 0) over the M x N output positions.
+// C <- beta * C (zero when beta == 0) over the M x N output positions.
 __global__ void __launch_bounds__(256) zcontract_scale_c(const ContractArgs a) {
   const int64_t total = a.M * a.N;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -319,24 +286,6 @@ __global__ void __launch_bounds__(256) zcontract_scale_c(const ContractArgs a) {
     double2* p = a.C + ocm + ocn;
     *p = a.beta_zero ? make_double2(0.0, 0.0) : cmul(a.beta, *p);
   }
-}
-
-int fill_modes(const ptn_modes& src, ModeDev& dst, int which, int64_t& total) {
-  // which: 0 -> (a, c) strides, 1 -> (b, c), 2 -> (a, b)
-  if (src.n < 0 || src.n > PTN_MAX_MODES) return PTN_ERR_ARG;
-  dst.n = src.n;
-  total = 1;
-  for (int i = 0; i < src.n; ++i) {
-    if (src.dim[i] <= 0) return PTN_ERR_ARG;
-    dst.dim[i] = src.dim[i];
-    total *= src.dim[i];
-    switch (which) {
-      case 0: dst.s0[i] = src.stride_a[i]; dst.s1[i] = src.stride_c[i]; break;
-      case 1: dst.s0[i] = src.stride_b[i]; dst.s1[i] = src.stride_c[i]; break;
-      default: dst.s0[i] = src.stride_a[i]; dst.s1[i] = src.stride_b[i]; break;
-    }
-  }
-  return PTN_OK;
 }
 
 }  // namespace
@@ -358,20 +307,8 @@ extern "C" int64_t ptn_zcontract_splits(int64_t tiles, int64_t K, int64_t* k_chu
 extern "C" int ptn_zcontract(const ptn_contract_desc* d, void* stream) {
   if (!d || !d->A || !d->B || !d->C) return PTN_ERR_ARG;
   ContractArgs a;
-  int64_t M, N, K;
-  if (fill_modes(d->m, a.m, 0, M) || fill_modes(d->n, a.n, 1, N) || fill_modes(d->k, a.k, 2, K))
-    return PTN_ERR_ARG;
-  a.A = static_cast<const double2*>(d->A);
-  a.B = static_cast<const double2*>(d->B);
-  a.C = static_cast<double2*>(d->C);
-  a.alpha = make_double2(d->alpha_re, d->alpha_im);
-  a.beta = make_double2(d->beta_re, d->beta_im);
-  a.beta_zero = (d->beta_re == 0.0 && d->beta_im == 0.0);
-  a.conj_a = d->conj_a;
-  a.conj_b = d->conj_b;
-  a.M = M;
-  a.N = N;
-  a.K = K;
+  if (zcontract_args(*d, a)) return PTN_ERR_ARG;
+  const int64_t M = a.M, N = a.N, K = a.K;
   if (M == 0 || N == 0) return PTN_OK;
   cudaStream_t s = ptn_stream(stream);
   if (M * N <= SMALL_MAX_OUT && K >= SMALL_MIN_K) {

@@ -240,14 +240,27 @@ class _NativeOps:
         check(_lib.load().ptn_exec_ops(self.ops, self.n, p, len(self.refs), _stream_ptr()), "ptn_exec_ops")
 
 
+def contract_work_bytes(desc, device) -> int:
+    """Device scratch a complex128 contraction takes to run on the tensor cores
+    (``ptn_zcontract_work_bytes``); 0: it runs on the FP64 units."""
+    if torch.device(device).type != "cuda":
+        return 0
+    return int(_lib.load().ptn_zcontract_work_bytes(ctypes.byref(desc)))
+
+
 class Plan:
     """A sequence of contraction steps with one dynamic input and output."""
 
     def __init__(self, ws: Workspace, steps, ws_sizes):
         self.ws = ws
         self.steps = steps
-        self.ws_sizes = ws_sizes  # name -> numel
+        self.ws_sizes = dict(ws_sizes)  # name -> numel
         self.flops = sum(s.flops for s in steps)
+        # scratch of the steps that run as digit products on the tensor cores
+        # (one slot: the steps run one after the other)
+        self.work = [contract_work_bytes(st.desc, ws.device) for st in steps]
+        if any(self.work):
+            self.ws_sizes["zc_work"] = (max(self.work) + 15) // 16
 
     def run(self, x_ptr: int = 0, y_ptr: int = 0):
         ws = self.ws
@@ -256,7 +269,9 @@ class Plan:
                 ws.get(name, n)
             self._sized_at = ws.gen     # slots only grow: still large enough until one is replaced
         if not hasattr(self, "_exec"):
-            self._exec = _NativeOps([(_lib.OP_ZCONTRACT, st.desc, st.refs) for st in self.steps])
+            self._exec = _NativeOps([(_lib.OP_ZCONTRACT_WS, st.desc, st.refs + (("ws", "zc_work"),)) if wb else
+                                     (_lib.OP_ZCONTRACT, st.desc, st.refs)
+                                     for st, wb in zip(self.steps, self.work)])
         self._exec.run(ws, x_ptr, y_ptr)
 
 

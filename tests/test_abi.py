@@ -52,3 +52,26 @@ def test_zcontract_split_rule_covers_k_exactly():
             assert (s - 1) * c < K <= s * c
             assert tiles * s <= 304 + tiles
             assert s == 1 or c >= 256 - 8
+
+
+def test_zcontract_scratch_rule():
+    """Scratch of the tensor-core complex128 path (host arithmetic): none below
+    its least size, and bounded by the digits of B, one GiB of digits of A (or
+    one row tile) and the partial sums."""
+    import ctypes
+    from pytreenet_gb300 import _lib
+    lib = _lib.load()
+
+    def need(M, N, K):
+        d = _lib.ContractDesc()
+        for g, n in ((d.m, M), (d.n, N), (d.k, K)):
+            g.n = 1
+            g.dim[0] = n
+        return int(lib.ptn_zcontract_work_bytes(ctypes.byref(d)))
+    assert need(16, 16, 16) == 0 and need(1, 1, 1) == 0
+    assert need(3000, 64, 64) == need(64, 3000, 64) > 0           # either operand may lead
+    for M, N, K in ((640, 128, 128), (1 << 22, 10, 10), (90, 31, 8100), (655360, 256, 1280)):
+        stages = (K + 15) // 16
+        a = max(1 << 30, stages * 57344)
+        b = (min(M, N) + 31) // 32 * stages * 28672
+        assert 0 < need(M, N, K) <= a + b + 16 * 152 * 128 * 64 + 16 * M + (1 << 24)
