@@ -6,8 +6,10 @@
 // working copy of A by plane rotations applied from the right; V accumulates
 // the rotations. A sweep visits every column pair once in the round-robin
 // (circle) order: n_even - 1 rounds of n_even / 2 disjoint pairs, one warp per
-// pair. Rounds are separated by a grid-wide barrier; the kernel is launched
-// cooperatively so all CTAs are resident. A pair (a, b) is rotated when
+// pair. Matrices of 8 columns and up to 512 rows run as a ring of CTAs that pass
+// columns to their neighbours (zsvd_ring_kernel); fewer columns in one CTA;
+// taller ones with rounds separated by a grid-wide barrier. Kernels whose CTAs
+// wait on one another are launched cooperatively, so all CTAs are resident. A pair (a, b) is rotated when
 // |a^H b| > tol * |a| |b| (tol = 8 sqrt(m) * 2^-53); the
 // iteration stops after the first sweep without a rotation. Every barrier wait
 // is bounded: on timeout the kernel records PTN_ERR_TIMEOUT in *status and all
@@ -181,13 +183,332 @@ __global__ void __launch_bounds__(SVD_THREADS) zsvd_jacobi_kernel(SvdArgs a) {
   }
 }
 
+// ---- ring of CTAs: one column pair each ----------------------------------------------------
+// The same sweeps, pairs and rotations as above without a grid barrier per
+// round. CTA p holds the columns at positions p and np - 1 - p of the circle;
+// from one round to the next a column moves one position, so it goes to the
+// neighbouring CTA (CTA 0 keeps position 0) and a round only waits for the two
+// neighbours. Columns travel through mailboxes in L2 (two per slot, by round
+// parity: a CTA sends its round-r columns only after it has the neighbour's of
+// round r - 1, which the neighbour sent after reading its mailbox of that
+// round). Every 8 bytes of a mailbox carry 4 bytes of the column and the number
+// of the round, so the reader polls the data themselves: no fence on either
+// side and one L2 round trip less than a separate flag (128 x 128: 7.3 ms with
+// flags and fences). Four warps hold the rows of A, four the rows of V; the
+// latter take each rotation from shared memory and stay out of the chain of
+// dependent rounds.
+//
+// What bounds it is the FP64 pipe (16 cycles per warp instruction on an SM,
+// whatever the active lanes) and the chain poll - dot - rotation - update - send
+// of a round. So the four sums of a pair are reduced together (six additions
+// instead of twenty), one warp forms the rotation, with two reciprocal square
+// roots: with d = |b|^2 - |a|^2, h = sqrt(d^2 + 4 |a^H b|^2), q = |d| + h,
+//   cos = q / sqrt(2 h q),  sin e^{i phi} = sign(d) 2 (a^H b) / sqrt(2 h q),
+// the smaller root as above; and the update is 12 FMAs per row. The matrix is
+// scaled by a power of two so that the squares stay in range. Measured: 128 x
+// 128 5.2 ms (18.2 ms with the grid barrier per round), 256 x 256 16.0 (61.0), 384
+// x 384 43.7 (123; more pairs than SMs).
+constexpr int RING_WARPS = 4;                        // per role: rows of A, rows of V
+constexpr int RING_ROWS = 32 * RING_WARPS;
+constexpr int RING_THREADS = 2 * RING_ROWS;
+constexpr int RING_MAX_R = 4;                        // rows per thread: m, n <= 512
+constexpr int64_t RING_MIN_N = 8;
+
+struct RingArgs {
+  SvdArgs a;
+  ulonglong2* box;          // [parity 2][CTA][slot 2][m + n][component 2]
+};
+
+// Sum over the warp of four values; every lane of quarter q (8 lanes) gets
+// value q.
+__device__ __forceinline__ double warp_sum4(double v0, double v1, double v2, double v3, int lane) {
+  const bool up = lane & 16;
+  const double k0 = up ? v2 : v0, k1 = up ? v3 : v1, s0 = up ? v0 : v2, s1 = up ? v1 : v3;
+  const double a = k0 + __shfl_xor_sync(0xffffffffu, s0, 16), b = k1 + __shfl_xor_sync(0xffffffffu, s1, 16);
+  const bool odd = lane & 8;
+  double r = (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
+  r += __shfl_xor_sync(0xffffffffu, r, 4);
+  r += __shfl_xor_sync(0xffffffffu, r, 2);
+  r += __shfl_xor_sync(0xffffffffu, r, 1);
+  return r;
+}
+
+// A mailbox entry: a component's low and high words, each in 8 bytes (one
+// access of the memory model) with the round's number above it.
+__device__ __forceinline__ ulonglong2 ld_mail(const ulonglong2* p) {
+  ulonglong2 v;
+  asm volatile("ld.volatile.global.v2.u64 {%0,%1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_mail1(ulonglong2* p, double v, unsigned long long round) {
+  asm volatile("st.volatile.global.v2.u64 [%0], {%1,%2};" ::"l"(p),
+               "l"(round | (unsigned)__double2loint(v)), "l"(round | (unsigned)__double2hiint(v))
+               : "memory");
+}
+__device__ __forceinline__ void st_mail(ulonglong2* p, double2 v, unsigned round) {
+  st_mail1(p, v.x, (unsigned long long)round << 32);
+  st_mail1(p + 1, v.y, (unsigned long long)round << 32);
+}
+__device__ __forceinline__ double mail_value(ulonglong2 v) { return __hiloint2double((int)v.y, (int)v.x); }
+
+// This thread's rows of two mailboxes once they carry `round`; a bounded wait
+// of the warp, false when the kernel must leave.
+template <int R>
+__device__ __forceinline__ bool ring_read(const ulonglong2* bx, const ulonglong2* by, int tid, int rows, unsigned round,
+                                          unsigned* ctrl, int32_t* status, double2* x, double2* y) {
+  const volatile unsigned* abort = ctrl + 2;
+  const long long t0 = clock64();
+  for (unsigned it = 1;; ++it) {
+    bool ok = true;
+    ulonglong2 v[R][4];
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      const int t = tid + RING_ROWS * u;
+      if (t < rows) {
+        v[u][0] = ld_mail(bx + 2 * t);
+        v[u][1] = ld_mail(bx + 2 * t + 1);
+        v[u][2] = ld_mail(by + 2 * t);
+        v[u][3] = ld_mail(by + 2 * t + 1);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      x[u] = y[u] = make_double2(0.0, 0.0);
+      if (tid + RING_ROWS * u < rows) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          ok = ok && (unsigned)(v[u][k].x >> 32) == round && (unsigned)(v[u][k].y >> 32) == round;
+        x[u] = make_double2(mail_value(v[u][0]), mail_value(v[u][1]));
+        y[u] = make_double2(mail_value(v[u][2]), mail_value(v[u][3]));
+      }
+    }
+    if (__all_sync(0xffffffffu, ok)) return true;
+    int give_up = 0;
+    if ((it & 63u) == 0u && *abort != 0u) give_up = 1;
+    if (clock64() - t0 > SVD_WAIT_CYCLES) {
+      atomicExch(ctrl + 2, 1u);
+      atomicCAS(status, 0, PTN_ERR_TIMEOUT);
+      give_up = 1;
+    }
+    if (__any_sync(0xffffffffu, give_up)) return false;
+  }
+}
+
+// R: rows per thread (128 R >= m >= n).
+template <int R>
+__global__ void __launch_bounds__(RING_THREADS) zsvd_ring_kernel(RingArgs g) {
+  const SvdArgs& a = g.a;
+  const int tid = threadIdx.x & (RING_ROWS - 1), lane = tid & 31, warp = tid >> 5;
+  const bool vrole = threadIdx.x >= RING_ROWS;       // rows of V
+  const int p = blockIdx.x, P = gridDim.x, m = (int)a.m, n = (int)a.n, np = 2 * P;
+  __shared__ double red[2][RING_WARPS][4];
+  __shared__ double rot[2][4];                       // cos, Re / Im of sin e^{i phi}, rotated?
+  __shared__ int s_fail;
+  if (threadIdx.x == 0) s_fail = 0;
+  const int64_t len = m + n;
+  const int rows = vrole ? n : m, off = vrole ? m : 0;
+  auto box = [&](unsigned par, int cta, int slot) {
+    return g.box + 2 * (((int64_t)(par & 1u) * 2 * P + 2 * cta + slot) * len + off);
+  };
+  // where the columns at this CTA's two positions go
+  const int to_x = p >= 2 ? p - 1 : 0, slot_x = p == 1 ? 1 : 0;
+  const int to_y = p + 1 < P ? p + 1 : p, slot_y = p + 1 < P ? 1 : (P == 1 ? 1 : 0);
+  const int cx = p, cy = np - 1 - p;                 // columns at the start of a sweep
+
+  // power of two above the largest component, then the largest column norm
+  int* top = reinterpret_cast<int*>(a.ctrl + 3);
+  auto src = [&](int c, int r) {
+    return (c < n && r < m) ? a.src[r * a.rs + c * a.cs] : make_double2(0.0, 0.0);
+  };
+  // rounds are numbered from 1: no mailbox carries one yet
+  for (unsigned par = 0; par < 2; ++par)
+    for (int t = tid; t < rows; t += RING_ROWS)
+      for (int k = 0; k < 4; ++k) box(par, p, k & 1)[2 * t + (k >> 1)] = make_ulonglong2(0ull, 0ull);
+  if (!vrole) {
+    int hi = 0;
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      const double2 x = src(cx, tid + RING_ROWS * u), y = src(cy, tid + RING_ROWS * u);
+      hi = max(hi, max(max(__double2hiint(x.x) & 0x7fffffff, __double2hiint(x.y) & 0x7fffffff),
+                       max(__double2hiint(y.x) & 0x7fffffff, __double2hiint(y.y) & 0x7fffffff)));
+    }
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0 && hi) atomicMax(top, hi);
+  }
+  if (!grid_barrier(a.ctrl, a.status)) return;
+  const int field = *((volatile int*)top) >> 20;
+  const bool scaled = field > 0 && field < 0x7fe;    // 2^(1023 - field) is a normal number
+  const double down = scaled ? __hiloint2double((2046 - field) << 20, 0) : 1.0;
+  const double upsc = scaled ? __hiloint2double(field << 20, 0) : 1.0;
+  unsigned long long* amax_bits = reinterpret_cast<unsigned long long*>(a.ctrl + 4);
+  double2 x[R], y[R];
+  // |column|^2 of x and y over the A rows: atomically into amax, or to sig
+  auto norms = [&](double& sx, double& sy) {
+    sx = sy = 0.0;
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      sx += cabs2(x[u]);
+      sy += cabs2(y[u]);
+    }
+    const double t = warp_sum4(sx, sy, 0.0, 0.0, lane);
+    if (!vrole && (lane & 7) == 0 && lane < 16) red[0][warp][lane >> 3] = t;
+    __syncthreads();
+    sx = sy = 0.0;
+    for (int w = 0; w < RING_WARPS; ++w) {
+      sx += red[0][w][0];
+      sy += red[0][w][1];
+    }
+  };
+  {
+    ulonglong2* bx = box(0, p, 0);
+    ulonglong2* by = box(0, p, 1);
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      const int r = tid + RING_ROWS * u;
+      x[u] = vrole ? make_double2(r == cx ? 1.0 : 0.0, 0.0) : cscale(src(cx, r), down);
+      y[u] = vrole ? make_double2(r == cy ? 1.0 : 0.0, 0.0) : cscale(src(cy, r), down);
+      if (r < rows) {
+        st_mail(bx + 2 * r, x[u], 1u);
+        st_mail(by + 2 * r, y[u], 1u);
+      }
+    }
+    double sx, sy;
+    norms(sx, sy);
+    if (threadIdx.x == 0) atomicMax(amax_bits, (unsigned long long)__double_as_longlong(sx > sy ? sx : sy));
+  }
+  if (!grid_barrier(a.ctrl, a.status)) return;
+  const double amax2 = __longlong_as_double((long long)*((volatile unsigned long long*)amax_bits));
+  const double tol2 = a.tol * a.tol, zero2 = tol2 * amax2;
+
+  unsigned done = 0;                                 // rounds completed
+  bool converged = (n < 2);
+  for (int sweep = 0; sweep < SVD_MAX_SWEEPS && !converged; ++sweep) {
+    unsigned count = 0;
+    for (int r = 0; r + 1 < np; ++r, ++done) {
+      const int ci = p == 0 ? 0 : 1 + (p - 1 + r) % (np - 1), cj = 1 + (np - 2 - p + r) % (np - 1);
+      const bool swap = ci > cj;                     // the lower column is the rotation's first
+      const int q = done & 1;
+      // (a warp that must leave tells the others at the round's barrier)
+      if (!ring_read<R>(box(done, p, swap ? 1 : 0), box(done, p, swap ? 0 : 1), tid, rows, done + 1, a.ctrl, a.status, x,
+                        y))
+        s_fail = 1;
+      if (!vrole) {
+        double al = 0.0, be = 0.0;
+        double2 ga = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+          al = fma(x[u].x, x[u].x, fma(x[u].y, x[u].y, al));
+          be = fma(y[u].x, y[u].x, fma(y[u].y, y[u].y, be));
+          ga = cfmac(x[u], y[u], ga);                // conj(x) y
+        }
+        const double part = warp_sum4(al, be, ga.x, ga.y, lane);
+        if ((lane & 7) == 0) red[q][warp][lane >> 3] = part;
+        asm volatile("bar.sync 1, %0;" ::"n"(RING_ROWS) : "memory");
+        if (warp == 0) {
+          double v = red[q][(lane >> 2) & 3][lane & 3];
+          v += __shfl_xor_sync(0xffffffffu, v, 4);
+          v += __shfl_xor_sync(0xffffffffu, v, 8);
+          al = __shfl_sync(0xffffffffu, v, 0);
+          be = __shfl_sync(0xffffffffu, v, 1);
+          ga.x = __shfl_sync(0xffffffffu, v, 2);
+          ga.y = __shfl_sync(0xffffffffu, v, 3);
+          const double g2 = fma(ga.x, ga.x, ga.y * ga.y);
+          const bool turn = al > zero2 && be > zero2 && g2 > tol2 * al * be;
+          double c = 1.0, sr = 0.0, si = 0.0;
+          if (turn) {
+            const double d = be - al, xx = fma(d, d, 4.0 * g2);
+            const double h = xx * rsqrt(xx), qq = fabs(d) + h, rr = rsqrt(2.0 * h * qq);
+            const double f = d >= 0.0 ? 2.0 * rr : -2.0 * rr;
+            c = qq * rr;
+            sr = f * ga.x;
+            si = f * ga.y;
+            ++count;
+          }
+          if (lane == 0) {
+            rot[q][0] = c;
+            rot[q][1] = sr;
+            rot[q][2] = si;
+            rot[q][3] = turn ? 1.0 : 0.0;
+          }
+        }
+      }
+      __syncthreads();
+      if (s_fail) return;
+      const double c = rot[q][0], sr = rot[q][1], si = rot[q][2];
+      const bool turn = rot[q][3] != 0.0;
+      ulonglong2* ox = box(done + 1, to_x, slot_x);
+      ulonglong2* oy = box(done + 1, to_y, slot_y);
+#pragma unroll
+      for (int u = 0; u < R; ++u) {
+        const int t = tid + RING_ROWS * u;
+        if (turn) {
+          // x <- c x - s e^{-i phi} y,  y <- s e^{i phi} x + c y
+          const double2 s = x[u], w = y[u];
+          x[u].x = fma(c, s.x, fma(-sr, w.x, -si * w.y));
+          x[u].y = fma(c, s.y, fma(-sr, w.y, si * w.x));
+          y[u].x = fma(c, w.x, fma(sr, s.x, -si * s.y));
+          y[u].y = fma(c, w.y, fma(sr, s.y, si * s.x));
+        }
+        if (t < rows) {
+          st_mail(ox + 2 * t, swap ? y[u] : x[u], done + 2);
+          st_mail(oy + 2 * t, swap ? x[u] : y[u], done + 2);
+        }
+      }
+    }
+    if (threadIdx.x == 0 && count) atomicAdd(a.ctrl + 8 + (sweep % (CTRL_WORDS - 8)), count);
+    if (!grid_barrier(a.ctrl, a.status)) return;
+    converged = *((volatile unsigned*)(a.ctrl + 8 + (sweep % (CTRL_WORDS - 8)))) == 0u;
+  }
+  if (!converged && p == 0 && threadIdx.x == 0) atomicCAS(a.status, 0, PTN_ERR_NOCONVERGE);
+
+  // norms, then every column to its place in descending order (as above)
+  {
+    if (!ring_read<R>(box(done, p, 0), box(done, p, 1), tid, rows, done + 1, a.ctrl, a.status, x, y)) s_fail = 1;
+    __syncthreads();
+    if (s_fail) return;
+    double sx, sy;
+    norms(sx, sy);
+    if (threadIdx.x == 0) {
+      __stcg(a.sig + cx, sqrt(sx));
+      if (cy < n) __stcg(a.sig + cy, sqrt(sy));
+    }
+  }
+  if (!grid_barrier(a.ctrl, a.status)) return;
+  for (int e = 0; e < 2; ++e) {
+    const int c = e ? cy : cx;
+    if (c >= n) continue;
+    // compared as bit patterns: the order of non-negative doubles, and a place
+    // of its own (first) for a column that is not a number
+    const double sj = __ldcg(a.sig + c);
+    const long long bj = __double_as_longlong(sj) & 0x7fffffffffffffffll;
+    int cnt = 0;
+    for (int i = lane; i < n; i += 32) {
+      const long long bi = __double_as_longlong(__ldcg(a.sig + i)) & 0x7fffffffffffffffll;
+      cnt += (bi > bj || (bi == bj && i < c)) ? 1 : 0;
+    }
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    const double inv = sj > 0.0 ? 1.0 / sj : 0.0;
+    double2* dst = vrole ? a.V + (int64_t)cnt * a.ldv : a.U + (int64_t)cnt * a.ldu;
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      const int t = tid + RING_ROWS * u;
+      const double2 v = e ? y[u] : x[u];
+      if (t < rows) dst[t] = vrole ? v : cscale(v, inv);
+    }
+    if (threadIdx.x == 0) a.S[cnt] = sj * upsc;
+  }
+}
+
 // ---- small matrices: one CTA, everything in shared memory --------------------------------
 // For n <= SVD_SMALL_N columns whose working copy and rotations fit in shared
-// memory (SVD_SMALL_BYTES) the same sweeps run in one CTA with CTA barriers
-// between rounds (no cooperative launch, no global traffic). Same pair
-// schedule, rotation formula, thresholds and ordering as the kernel above, one
-// warp per pair (the pairs of a round are disjoint, so how they are spread over
-// the warps does not matter), so the results are the same bit for bit.
+// memory (SVD_SMALL_BYTES) and that the ring does not take (n < 8, or more than
+// 512 rows) the same sweeps run in one CTA with CTA barriers between rounds (no
+// cooperative launch, no global traffic): 86 us for 5 x 3. From 8 columns on one
+// SM's FP64 pipe is the bound (8 x 8 296 us, ring 177 us; 32 x 32 5.4 ms, ring 0.90
+// ms; 64 x 64 28.4 ms, ring 2.0 ms). Same pair schedule, rotation formula,
+// thresholds and ordering as zsvd_jacobi_kernel, one warp per pair (the pairs of
+// a round are disjoint, so how they are spread over the warps does not matter),
+// so the results are the same bit for bit.
 constexpr int64_t SVD_SMALL_N = 64;
 constexpr int64_t SVD_SMALL_BYTES = 200 * 1024;
 constexpr int SVD_SMALL_THREADS = 1024;
@@ -314,21 +635,33 @@ __global__ void __launch_bounds__(SVD_SMALL_THREADS) zsvd_jacobi_small_kernel(Sv
   }
 }
 
-int g_svd_max_blocks[64] = {0};
+// Co-resident CTAs of a kernel on the current device (kernel: an index into the
+// table, one per cooperative kernel).
+constexpr int SVD_KERNELS = 1 + RING_MAX_R;
+int g_svd_max_blocks[64][SVD_KERNELS] = {};
 std::mutex g_svd_mutex;
 
-int svd_max_blocks() {
+int svd_max_blocks(int kernel, const void* fn, int threads) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
   std::lock_guard<std::mutex> lock(g_svd_mutex);
-  if (g_svd_max_blocks[dev] == 0) {
+  int& cached = g_svd_max_blocks[dev][kernel];
+  if (cached == 0) {
     int per_sm = 0, sms = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, zsvd_jacobi_kernel, SVD_THREADS, 0) != cudaSuccess)
-      return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, 0) != cudaSuccess) return 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    g_svd_max_blocks[dev] = per_sm * sms;
+    cached = per_sm * sms;
   }
-  return g_svd_max_blocks[dev];
+  return cached;
+}
+
+const void* ring_kernel(int r) {
+  switch (r) {
+    case 1: return (const void*)zsvd_ring_kernel<1>;
+    case 2: return (const void*)zsvd_ring_kernel<2>;
+    case 3: return (const void*)zsvd_ring_kernel<3>;
+    default: return (const void*)zsvd_ring_kernel<4>;
+  }
 }
 
 inline int64_t align256(int64_t x) { return (x + 255) & ~int64_t(255); }
@@ -357,7 +690,10 @@ __global__ void zpermute_kernel(ptn_permute_desc d, int64_t total) {
 
 extern "C" int64_t ptn_zsvd_work_bytes(int64_t m, int64_t n) {
   if (m < 1 || n < 1) return 0;
-  return CTRL_BYTES + align256(16 * m * n) + align256(16 * n * n) + align256(8 * n);
+  // control words, norms, then the working copies of the columns (in the ring
+  // two mailboxes each, of twice a column's size)
+  const int64_t np = (n + 1) & ~int64_t(1);
+  return CTRL_BYTES + align256(8 * n) + align256((n >= RING_MIN_N && m <= RING_MAX_R * RING_ROWS ? 64 : 16) * np * (m + n));
 }
 
 extern "C" int ptn_zsvd_jacobi(const ptn_svd_desc* d, void* stream) {
@@ -370,10 +706,12 @@ extern "C" int ptn_zsvd_jacobi(const ptn_svd_desc* d, void* stream) {
   a.m = d->m;
   a.n = d->n;
   uint8_t* w = static_cast<uint8_t*>(d->work);
+  const int64_t np = (d->n + 1) & ~int64_t(1);
   a.ctrl = reinterpret_cast<unsigned*>(w);
-  a.Aw = reinterpret_cast<double2*>(w + CTRL_BYTES);
-  a.Vw = reinterpret_cast<double2*>(w + CTRL_BYTES + align256(16 * d->m * d->n));
-  a.sig = reinterpret_cast<double*>(w + CTRL_BYTES + align256(16 * d->m * d->n) + align256(16 * d->n * d->n));
+  a.sig = reinterpret_cast<double*>(w + CTRL_BYTES);
+  double2* cols = reinterpret_cast<double2*>(w + CTRL_BYTES + align256(8 * d->n));
+  a.Aw = cols;
+  a.Vw = cols + d->m * d->n;
   a.U = static_cast<double2*>(d->U);
   a.ldu = d->ldu;
   a.S = d->S;
@@ -385,6 +723,21 @@ extern "C" int ptn_zsvd_jacobi(const ptn_svd_desc* d, void* stream) {
   a.tol = 8.0 * sqrt((double)d->m) * 1.1102230246251565e-16;
   a.status = d->status;
   cudaStream_t s = ptn_stream(stream);
+  const int r = (int)((d->m + RING_ROWS - 1) / RING_ROWS);
+  if (d->n >= RING_MIN_N && r <= RING_MAX_R && np / 2 <= svd_max_blocks(r, ring_kernel(r), RING_THREADS)) {
+    if (cudaMemsetAsync(a.ctrl, 0, CTRL_BYTES, s) != cudaSuccess) return PTN_ERR_LAUNCH;
+    RingArgs g;
+    g.a = a;
+    g.box = reinterpret_cast<ulonglong2*>(cols);
+    void* args[] = {&g};
+    PTN_COUNT(1);
+    if (cudaLaunchCooperativeKernel(ring_kernel(r), dim3((unsigned)(np / 2)), dim3(RING_THREADS), args, 0, s) !=
+        cudaSuccess) {
+      cudaGetLastError();
+      return PTN_ERR_LAUNCH;
+    }
+    return PTN_OK;
+  }
   const size_t smem = (size_t)(d->m * d->n + d->n * d->n) * sizeof(double2);
   if (d->n <= SVD_SMALL_N && smem <= (size_t)SVD_SMALL_BYTES) {
     static const cudaError_t attr = cudaFuncSetAttribute(
@@ -394,7 +747,7 @@ extern "C" int ptn_zsvd_jacobi(const ptn_svd_desc* d, void* stream) {
     zsvd_jacobi_small_kernel<<<1, SVD_SMALL_THREADS, smem, s>>>(a);
     return ptn_launch_status();
   }
-  const int maxb = svd_max_blocks();
+  const int maxb = svd_max_blocks(0, (const void*)zsvd_jacobi_kernel, SVD_THREADS);
   if (maxb <= 0) return PTN_ERR_LAUNCH;
   if (cudaMemsetAsync(a.ctrl, 0, CTRL_BYTES, s) != cudaSuccess) return PTN_ERR_LAUNCH;
   const int64_t pairs = (((d->n + 1) & ~int64_t(1)) / 2);
