@@ -11,12 +11,15 @@
 // steps of 8. Tile offsets of the M and N rows are decoded once per CTA; the K
 // offsets once per K step.
 //
-// Skinny outputs over a long K (an environment, or the gradient of one, is
+// Outputs of less than 152 tiles run on zcontract_elem_kernel. Skinny outputs of
+// more than 4096 entries over a long K (an environment, or the gradient of one, is
 // chi x w x chi summed over everything else) would leave most SMs idle with
 // one CTA per output tile, so when there are few tiles the K range is split
 // over gridDim.y: a first kernel writes beta * C (or zero), and each split
 // adds alpha times its partial sums with double-precision atomics. The
 // summation order then varies between runs at the level of rounding.
+#include <cooperative_groups.h>
+
 #include "ptn_common.cuh"
 #include "zmodes.cuh"
 
@@ -125,102 +128,30 @@ __global__ void __launch_bounds__(256) zcontract_kernel(const ContractArgs a) {
   }
 }
 
-// Few outputs over a long K (a reduced density matrix: 2 x 2 outputs summed
-// over every bond index; the last step of a small environment update): the
-// tiled kernel would walk K on one CTA in steps of BK. Here each output is
-// summed by a group of G = SMALL_THREADS / P threads (P = the next power of two
-// of M * N), lane g of the group taking k = g, g + G, ...; the group's partial
-// sums are then added by a fixed tree, so the result does not vary between runs.
-constexpr int SMALL_THREADS = 1024;
-constexpr int64_t SMALL_MAX_OUT = 256;   // M * N up to this (G >= 4)
-constexpr int64_t SMALL_MIN_K = 64;
+// Products with fewer output tiles than SMs: the tiled kernel would put a whole
+// 64 x 64 tile -- most of it padding when M or N is small -- on each of a few SMs,
+// at ~2 FP64 FMAs per clock per SM. Here one thread sums one output over one of S
+// interleaved K slices (S = 1, 2, ..., 32) of a CTA, and for long K a cluster of C
+// CTAs (up to 8) takes K in equal ranges, so that few outputs still reach the FP64
+// units of many SMs; CTAs have four warps, one per scheduler and its FP64 unit.
+// The slices are added in order and the CTAs' sums by the first CTA in order,
+// through distributed shared memory: the result does not vary between runs. The
+// K offsets are decoded once per CTA into shared memory. Measured against one
+// thread per output and, for up to 256 outputs, one CTA of 1024 threads: 128 x 64,
+// K = 64 16.5 -> 10 us; 64 x 64, K = 128 29 -> 10; 13 x 13, K = 1014 186 -> 12;
+// 2 x 2, K = 4096 39 -> 12 (all with ~7 us of host call).
+constexpr int ELEM_THREADS = 128;
+constexpr int ELEM_MAX_CLUSTER = 8;
+constexpr int64_t ELEM_SPLIT_OUT = 4096;   // outputs up to which K ranges go to clusters
 
-__global__ void __launch_bounds__(SMALL_THREADS) zcontract_small_kernel(const ContractArgs a) {
-  __shared__ double2 part[SMALL_THREADS];
-  __shared__ int64_t offAk[SMALL_THREADS], offBk[SMALL_THREADS];
-  const int tid = threadIdx.x;
-  const int64_t outs = a.M * a.N;
-  int P = 1;
-  while (P < outs) P <<= 1;
-  const int G = SMALL_THREADS / P;
-  const int o = tid / G, g = tid - o * G;
-  double2 acc = make_double2(0.0, 0.0);
-  int64_t oa = 0, ob = 0, ocm = 0, ocn = 0;
-  if (o < outs) {
-    const int64_t mi = o / a.N, ni = o - mi * a.N;
-    decode(a.m, mi, oa, ocm);
-    decode(a.n, ni, ob, ocn);
-  }
-  // the K offsets of a chunk of SMALL_THREADS indices are decoded once, one
-  // per thread; each lane still takes k = g, g + G, ... in increasing order
-  // (G divides the chunk)
-  for (int64_t k0 = 0; k0 < a.K; k0 += SMALL_THREADS) {
-    {
-      const int64_t k = k0 + tid;
-      int64_t x = 0, y = 0;
-      if (k < a.K) decode(a.k, k, x, y);
-      offAk[tid] = x;
-      offBk[tid] = y;
-    }
-    __syncthreads();
-    if (o < outs) {
-      const int cnt = (int)(a.K - k0 < SMALL_THREADS ? a.K - k0 : SMALL_THREADS);
-      // eight operand pairs loaded ahead of their (in-order) accumulation, so
-      // the loads overlap; the order of the additions is unchanged
-      constexpr int AHEAD = 8;
-      int kk = g;
-      for (; kk + (AHEAD - 1) * G < cnt; kk += AHEAD * G) {
-        double2 x[AHEAD], y[AHEAD];
-#pragma unroll
-        for (int u = 0; u < AHEAD; ++u) {
-          x[u] = a.A[oa + offAk[kk + u * G]];
-          y[u] = a.B[offBk[kk + u * G] + ob];
-        }
-#pragma unroll
-        for (int u = 0; u < AHEAD; ++u) {
-          if (a.conj_a) x[u].y = -x[u].y;
-          if (a.conj_b) y[u].y = -y[u].y;
-          acc = cfma(x[u], y[u], acc);
-        }
-      }
-      for (; kk < cnt; kk += G) {
-        double2 x = a.A[oa + offAk[kk]];
-        double2 y = a.B[offBk[kk] + ob];
-        if (a.conj_a) x.y = -x.y;
-        if (a.conj_b) y.y = -y.y;
-        acc = cfma(x, y, acc);
-      }
-    }
-    __syncthreads();
-  }
-  part[tid] = acc;
-  __syncthreads();
-  for (int h = G / 2; h > 0; h >>= 1) {
-    if (g < h) {
-      const double2 u = part[tid + h];
-      part[tid] = make_double2(part[tid].x + u.x, part[tid].y + u.y);
-    }
-    __syncthreads();
-  }
-  if (g == 0 && o < outs) {
-    double2* p = a.C + ocm + ocn;
-    double2 v = cmul(a.alpha, part[tid]);
-    if (!a.beta_zero) v = cfma(a.beta, *p, v);
-    *p = v;
-  }
-}
-
-// Products with fewer output tiles than SMs (and no K split): the tiled
-// kernel would put a whole 64 x 64 tile -- most of it padding when M or N is
-// small -- on each of a few SMs, at ~2 FP64 FMAs per clock per SM. Here one
-// thread owns one output and adds A[m, k] B[k, n] over k in increasing order
-// with the same complex FMA as the tiled kernel, so the result has the same
-// bits; the K offsets are decoded once per CTA into shared memory.
-constexpr int ELEM_THREADS = 64;
-
-__global__ void __launch_bounds__(ELEM_THREADS) zcontract_elem_kernel(const ContractArgs a) {
+template <int S>
+__global__ void __launch_bounds__(ELEM_THREADS) zcontract_elem_kernel(const ContractArgs a, const int C) {
+  constexpr int OUTS = ELEM_THREADS / S;             // outputs per cluster
   __shared__ int64_t offAk[ELEM_THREADS], offBk[ELEM_THREADS];
-  const int64_t o = blockIdx.x * (int64_t)ELEM_THREADS + threadIdx.x;
+  __shared__ double2 part[ELEM_THREADS];
+  const int rank = C > 1 ? (int)(blockIdx.x % C) : 0;
+  const int slice = threadIdx.x / OUTS;
+  const int64_t o = (blockIdx.x / C) * (int64_t)OUTS + (threadIdx.x - slice * OUTS);
   const bool valid = o < a.M * a.N;
   int64_t oa = 0, ocm = 0, ob = 0, ocn = 0;
   if (valid) {
@@ -229,26 +160,27 @@ __global__ void __launch_bounds__(ELEM_THREADS) zcontract_elem_kernel(const Cont
     decode(a.n, ni, ob, ocn);
   }
   double2 acc = make_double2(0.0, 0.0);
-  for (int64_t k0 = 0; k0 < a.K; k0 += ELEM_THREADS) {
-    __syncthreads();
+  const int64_t kbeg = rank * a.k_chunk, kend = kbeg + a.k_chunk < a.K ? kbeg + a.k_chunk : a.K;
+  for (int64_t k0 = kbeg; k0 < kend; k0 += ELEM_THREADS) {
+    if (k0 != kbeg) __syncthreads();
     {
       const int64_t k = k0 + threadIdx.x;
-      int64_t x = -1, y = -1;
-      if (k < a.K) decode(a.k, k, x, y);
+      int64_t x = 0, y = 0;
+      if (k < kend) decode(a.k, k, x, y);
       offAk[threadIdx.x] = x;
       offBk[threadIdx.x] = y;
     }
     __syncthreads();
-    const int cnt = (int)(a.K - k0 < ELEM_THREADS ? a.K - k0 : ELEM_THREADS);
+    const int cnt = (int)(kend - k0 < ELEM_THREADS ? kend - k0 : ELEM_THREADS);
     if (valid) {
       // operand pairs loaded four ahead of their in-order accumulation
-      int kk = 0;
-      for (; kk + 3 < cnt; kk += 4) {
+      int kk = slice;
+      for (; kk + 3 * S < cnt; kk += 4 * S) {
         double2 av[4], bv[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          av[u] = a.A[oa + offAk[kk + u]];
-          bv[u] = a.B[offBk[kk + u] + ob];
+          av[u] = a.A[oa + offAk[kk + u * S]];
+          bv[u] = a.B[offBk[kk + u * S] + ob];
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -257,7 +189,7 @@ __global__ void __launch_bounds__(ELEM_THREADS) zcontract_elem_kernel(const Cont
           acc = cfma(av[u], bv[u], acc);
         }
       }
-      for (; kk < cnt; ++kk) {
+      for (; kk < cnt; kk += S) {
         double2 av = a.A[oa + offAk[kk]];
         double2 bv = a.B[offBk[kk] + ob];
         if (a.conj_a) av.y = -av.y;
@@ -266,7 +198,23 @@ __global__ void __launch_bounds__(ELEM_THREADS) zcontract_elem_kernel(const Cont
       }
     }
   }
-  if (valid) {
+  if (S > 1) {
+    part[threadIdx.x] = acc;
+    __syncthreads();
+    if (slice == 0)
+      for (int u = 1; u < S; ++u) acc = cadd(acc, part[threadIdx.x + u * OUTS]);
+  }
+  if (C > 1) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    if (slice == 0) part[threadIdx.x] = acc;
+    cluster.sync();
+    if (rank == 0 && slice == 0)
+      for (int r = 1; r < C; ++r) acc = cadd(acc, cluster.map_shared_rank(part, r)[threadIdx.x]);
+    cluster.sync();                                  // the others' shared memory was being read
+    if (rank != 0) return;
+  }
+  if (valid && slice == 0) {
     double2* p = a.C + ocm + ocn;
     double2 v = cmul(a.alpha, acc);
     if (!a.beta_zero) v = cfma(a.beta, *p, v);
@@ -285,6 +233,64 @@ __global__ void __launch_bounds__(256) zcontract_scale_c(const ContractArgs a) {
     decode(a.n, ni, ob, ocn);
     double2* p = a.C + ocm + ocn;
     *p = a.beta_zero ? make_double2(0.0, 0.0) : cmul(a.beta, *p);
+  }
+}
+
+template <int S>
+int64_t launch_elem_s(ContractArgs& a, int c, cudaStream_t s) {
+  constexpr int64_t outs = ELEM_THREADS / S;
+  const int64_t blocks = (a.M * a.N + outs - 1) / outs * c;
+  if (blocks > 0x7fffffffLL) return 0;
+  a.k_chunk = (a.K + c - 1) / c;
+  PTN_COUNT(1);
+  if (c == 1) {
+    zcontract_elem_kernel<S><<<(unsigned)blocks, ELEM_THREADS, 0, s>>>(a, c);
+    return blocks;
+  }
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)c;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3(ELEM_THREADS);
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, zcontract_elem_kernel<S>, a, c) != cudaSuccess) {
+    cudaGetLastError();
+    return -1;
+  }
+  return blocks;
+}
+
+// The launch of zcontract_elem_kernel. K slices: the count with the least FP64
+// time on the fullest SM (CTAs per SM, rounded up, times the k of a slice, plus
+// the adding up), at least eight k each; then, for few outputs, a cluster over
+// ranges of K. Returns the CTAs launched, 0 when the outputs are too many, -1 on
+// an error.
+int64_t launch_elem(ContractArgs& a, cudaStream_t s) {
+  const int64_t out = a.M * a.N;
+  int sl = 1, c = 1;
+  int64_t best = INT64_MAX;
+  for (int t = 1; t <= 32 && (t == 1 || a.K >= 8 * t); t *= 2) {
+    const int64_t blocks = (out * t + ELEM_THREADS - 1) / ELEM_THREADS;
+    const int64_t cost = (blocks + 151) / 152 * (4 * ((a.K + t - 1) / t) + 8 + t / 2);
+    if (cost < best) {
+      best = cost;
+      sl = t;
+    }
+  }
+  while (out <= ELEM_SPLIT_OUT && sl == 32 && c < ELEM_MAX_CLUSTER && out * sl * c < 152 * ELEM_THREADS &&
+         a.K >= 16 * sl * c)
+    c *= 2;
+  switch (sl) {
+    case 1: return launch_elem_s<1>(a, c, s);
+    case 2: return launch_elem_s<2>(a, c, s);
+    case 4: return launch_elem_s<4>(a, c, s);
+    case 8: return launch_elem_s<8>(a, c, s);
+    case 16: return launch_elem_s<16>(a, c, s);
+    default: return launch_elem_s<32>(a, c, s);
   }
 }
 
@@ -311,27 +317,15 @@ extern "C" int ptn_zcontract(const ptn_contract_desc* d, void* stream) {
   const int64_t M = a.M, N = a.N, K = a.K;
   if (M == 0 || N == 0) return PTN_OK;
   cudaStream_t s = ptn_stream(stream);
-  if (M * N <= SMALL_MAX_OUT && K >= SMALL_MIN_K) {
-    a.tiles_n = 1;
-    a.k_chunk = K;
-    a.split = 0;
-    PTN_COUNT(1);
-    zcontract_small_kernel<<<1, SMALL_THREADS, 0, s>>>(a);
-    return ptn_launch_status();
-  }
   int64_t tm = (M + BM - 1) / BM, tn = (N + BN - 1) / BN;
   a.tiles_n = tn;
   int64_t tiles = tm * tn;
   if (tiles > 0x7fffffffLL) return PTN_ERR_UNSUPPORTED;
   int64_t splits = ptn_zcontract_splits(tiles, K, &a.k_chunk);
   a.split = splits > 1;
-  if (!a.split && tiles < 152) {
-    const int64_t blocks = (M * N + ELEM_THREADS - 1) / ELEM_THREADS;
-    if (blocks <= 0x7fffffffLL) {
-      PTN_COUNT(1);
-      zcontract_elem_kernel<<<(unsigned)blocks, ELEM_THREADS, 0, s>>>(a);
-      return ptn_launch_status();
-    }
+  if (tiles < 152 && (!a.split || M * N <= ELEM_SPLIT_OUT)) {
+    const int64_t blocks = launch_elem(a, s);
+    if (blocks != 0) return blocks > 0 ? ptn_launch_status() : PTN_ERR_LAUNCH;
   }
   if (a.split) {
     int64_t total = M * N;
