@@ -345,6 +345,44 @@ int ptn_exec_ops(const ptn_exec_op* ops, int32_t nops, void* const* ptrs, int32_
 int ptn_krylov_gs_step(const void* Q, int64_t ldq, int32_t nq, void* w, int64_t n, void* h,
                        void* partial, double* norms, void* qnext, void* stream);
 
+/* A batch of steps of krylov_exp_action (time_evolution/time_evolution.py:721-821)
+ * on the operator given as a plan: for j0 <= j < j0 + batch the plan runs from
+ * basis row j into w, followed by one Gram-Schmidt step; then the coefficients
+ * come to the host in one synchronisation and the reference's decisions are
+ * taken there (happy breakdown, the stop beta0 beta |exp(z T) e_1|_m < tol, the
+ * basis capacity). With j0 = 0 the batch begins with beta0 = |x| and row 0 =
+ * x / beta0. Outputs: m (steps that count), done, and after done the column
+ * beta0 exp(z T_m) e_1 in coef, which ptn_krylov_combine writes out as
+ * out = sum_i coef_i Q_i. T (host, ldt x ldt complex128) keeps the projection
+ * between batches: column j holds the coefficients of step j, its subdiagonal
+ * |w|. Host memory that the device copies into is pinned. All other pointers
+ * are device memory. beta0 = 0 returns done with m = 0. PTN_ERR_NONFINITE for a
+ * vector that is not finite; a nonzero *status_host is left to the caller. */
+typedef struct {
+  const ptn_exec_op* ops;
+  int32_t nops, nptrs;
+  void** ptrs;              /* table of the plan; entries 0 and 1 are set here  */
+  const void* x;            /* read when j0 = 0                                 */
+  void* Q;                  /* qcap rows of n                                   */
+  void* w;                  /* n                                                */
+  void* h;                  /* complex128[J (J + 1)], J = j0 + batch            */
+  void* norms;              /* double[1 + 2 J]                                  */
+  void* partial;            /* ptn_krylov_partials(n)                           */
+  const int32_t* status;    /* device status word of the plan, or null          */
+  void* h_host;             /* pinned, as h                                     */
+  double* norms_host;       /* pinned, as norms                                 */
+  int32_t* status_host;     /* pinned                                           */
+  void* T;
+  void* coef;               /* host, complex128[j0 + batch]                     */
+  int64_t n, ldt;
+  int32_t qcap, j0, batch, tridiagonal;
+  double z_re, z_im, tol;
+  double beta0;             /* out with j0 = 0, in afterwards                   */
+  int32_t m, done;          /* out                                              */
+} ptn_krylov_desc;
+int ptn_krylov_batch(ptn_krylov_desc* d, void* stream);
+int ptn_krylov_combine(const void* Q, int64_t n, int32_t m, const void* coef_host, void* out, void* stream);
+
 unsigned long long ptn_launch_counter(void);
 
 /* Wait until all work issued on `stream` has finished (cudaStreamSynchronize);

@@ -88,6 +88,18 @@ class ExecOp(ctypes.Structure):
                 ("desc", ctypes.c_void_p)]
 
 
+class KrylovDesc(ctypes.Structure):
+    _fields_ = [("ops", ctypes.POINTER(ExecOp)), ("nops", ctypes.c_int32), ("nptrs", ctypes.c_int32),
+                ("ptrs", ctypes.POINTER(ctypes.c_void_p)), ("x", ctypes.c_void_p), ("Q", ctypes.c_void_p),
+                ("w", ctypes.c_void_p), ("h", ctypes.c_void_p), ("norms", ctypes.c_void_p),
+                ("partial", ctypes.c_void_p), ("status", ctypes.c_void_p), ("h_host", ctypes.c_void_p),
+                ("norms_host", ctypes.c_void_p), ("status_host", ctypes.c_void_p), ("T", ctypes.c_void_p),
+                ("coef", ctypes.c_void_p), ("n", ctypes.c_int64), ("ldt", ctypes.c_int64),
+                ("qcap", ctypes.c_int32), ("j0", ctypes.c_int32), ("batch", ctypes.c_int32),
+                ("tridiagonal", ctypes.c_int32), ("z_re", ctypes.c_double), ("z_im", ctypes.c_double),
+                ("tol", ctypes.c_double), ("beta0", ctypes.c_double), ("m", ctypes.c_int32), ("done", ctypes.c_int32)]
+
+
 OP_ZCONTRACT, OP_CGEMM, OP_TO_PLANES, OP_EXPAND_B, OP_ZCONTRACT_WS = 0, 1, 2, 3, 4
 
 _P = ctypes.c_void_p
@@ -131,6 +143,8 @@ SIGNATURES = {
     "ptn_zsvd_jacobi": (ctypes.c_int, [ctypes.POINTER(SvdDesc), _P]),
     "ptn_zpermute": (ctypes.c_int, [ctypes.POINTER(PermuteDesc), _P]),
     "ptn_exec_ops": (ctypes.c_int, [ctypes.POINTER(ExecOp), _I32, ctypes.POINTER(ctypes.c_void_p), _I32, _P]),
+    "ptn_krylov_batch": (ctypes.c_int, [ctypes.POINTER(KrylovDesc), _P]),
+    "ptn_krylov_combine": (ctypes.c_int, [_P, _I64, _I32, _P, _P, _P]),
     "ptn_krylov_gs_step": (ctypes.c_int, [_P, _I64, _I32, _P, _I64, _P, _P, _P, _P, _P]),
 }
 

@@ -40,6 +40,7 @@ subtree dimensions): the QR of a rank-deficient matrix has no derivative.
 from __future__ import annotations
 
 import ctypes
+import threading
 from typing import Callable
 
 import numpy as np
@@ -236,33 +237,84 @@ def bond_apply(r, e_q, e_n, batch=False, out=None):
 class _SiteOp:
     def __init__(self, n):
         self.n = n
+        self.key = ("site", n)
 
     def apply(self, x, params, batch=False, out=None):
         return site_apply(x, list(params[:self.n]), params[self.n], batch=batch, out=out)
 
+    def chain(self, cb, x_shape, params):
+        """``site_apply`` as a contraction chain over the operands ``params``
+        (environments, then W), each made by ``params[i](labels)``."""
+        n = self.n
+        half = n // 2
+        T = Operand.contiguous(("in",), [f"a{k}" for k in range(n)] + ["s"], list(x_shape))
+        for k in range(half):
+            T = cb.contract(T, params[k]([f"a{k}", f"b{k}", f"c{k}"]), [f"a{k}"])
+        T = cb.contract(T, params[n]([f"b{k}" for k in range(n)] + ["t", "s"]), [f"b{k}" for k in range(half)] + ["s"])
+        y = Operand.contiguous(("out",), [f"c{k}" for k in range(n)] + ["t"], list(x_shape))
+        for k in range(half, n):
+            T = cb.contract(T, params[k]([f"a{k}", f"b{k}", f"c{k}"]), [f"a{k}", f"b{k}"],
+                            out=y if k == n - 1 else None)
+
 
 class _BondOp:
+    key = ("bond",)
+
     def apply(self, x, params, batch=False, out=None):
         return bond_apply(x, params[0], params[1], batch=batch, out=out)
+
+    def chain(self, cb, x_shape, params):
+        r = Operand.contiguous(("in",), ["a", "c"], list(x_shape))
+        T = cb.contract(params[0](["a", "b", "x"]), r, ["a"])
+        cb.contract(T, params[1](["c", "b", "y"]), ["c", "b"],
+                    out=Operand.contiguous(("out",), ["x", "y"], list(x_shape)))
 
 
 # ----------------------------------------------------------------------------
 # Krylov exponential and its adjoint
 # ----------------------------------------------------------------------------
-_SOLVERS: dict = {}
+_SOLVERS = threading.local()
+OP_PLANS_KEPT = 256            # operator plans per solver (kinds and shapes)
 
 
 def _solver(device) -> KrylovSolver:
+    """The calling thread's solver on ``device`` (its workspace holds the basis
+    and the vectors of the solve that runs)."""
+    per_device = _SOLVERS.__dict__.setdefault("solvers", {})
     key = str(device)
-    if key not in _SOLVERS:
-        _SOLVERS[key] = KrylovSolver(Workspace(torch.device(device)))
-    return _SOLVERS[key]
+    if key not in per_device:
+        per_device[key] = KrylovSolver(Workspace(torch.device(device)))
+        per_device[key].op_plans = {}
+    return per_device[key]
+
+
+def _operator_plan(solver, op, params, shape):
+    """``op`` on ``params`` as a complex128 plan: built once per kind and shapes,
+    its operands' addresses set here for the solve that follows."""
+    key = (op.key, tuple(shape), tuple(tuple(p.shape) for p in params))
+    ent = solver.op_plans.get(key)
+    if ent is None:
+        if len(solver.op_plans) >= OP_PLANS_KEPT:
+            solver.op_plans.pop(next(iter(solver.op_plans)))
+        holders = [_Ptr() for _ in params]
+        cb = E.ChainBuilder(solver.ws)
+        op.chain(cb, shape, [lambda labels, h=h, p=p: Operand.contiguous(("fixed", h), labels, list(p.shape))
+                             for h, p in zip(holders, params)])
+        ent = solver.op_plans[key] = (cb.plan(), holders)
+    plan, holders = ent
+    for h, p in zip(holders, params):
+        h.p = p.data_ptr()
+    return plan
 
 
 def _tensor_apply(op, params, shape):
     def ap(xq, w):
         op.apply(xq.view(shape), params, out=w.view(shape))
     ap.takes_tensors = True
+    if not _LEVELS["levels"] and params[0].device.type == "cuda":
+        # contiguous copies, if any, live as long as this operator
+        ap.params = params = [p.contiguous() for p in params]
+        ap.plan = _operator_plan(_solver(params[0].device), op, params, shape)
     return ap
 
 

@@ -145,6 +145,7 @@ def effective_single_site_evolution(state_tensor, state_node, hamiltonian_tensor
 
     def apply(xp, yp):
         p.run(xp, yp)
+    apply.plan = p
     out = torch.empty_like(x)
     ode = ode_options(mode, options)
     if ode is not None:

@@ -224,9 +224,9 @@ class _NativeOps:
         self._moving = [i for i in range(2, len(self.refs))
                         if self.refs[i][0] == "fixed" and not isinstance(self.refs[i][1], torch.Tensor)]
 
-    def run(self, ws, x_ptr, y_ptr):
+    def bind(self, ws):
+        """The pointer table, current except for the input and the output."""
         p = self.ptrs
-        p[0], p[1] = x_ptr or None, y_ptr or None
         # fixed tensors never move, workspace slots only when the workspace's
         # generation changed since the table was last filled
         if self._gen != ws.gen:
@@ -237,6 +237,11 @@ class _NativeOps:
         else:
             for i in self._moving:
                 p[i] = self.refs[i][1].data_ptr()
+        return p
+
+    def run(self, ws, x_ptr, y_ptr):
+        p = self.bind(ws)
+        p[0], p[1] = x_ptr or None, y_ptr or None
         check(_lib.load().ptn_exec_ops(self.ops, self.n, p, len(self.refs), _stream_ptr()), "ptn_exec_ops")
 
 
@@ -262,7 +267,8 @@ class Plan:
         if any(self.work):
             self.ws_sizes["zc_work"] = (max(self.work) + 15) // 16
 
-    def run(self, x_ptr: int = 0, y_ptr: int = 0):
+    def native_ops(self) -> "_NativeOps":
+        """The plan's launch list, its workspace slots allocated."""
         ws = self.ws
         if getattr(self, "_sized_at", None) != ws.gen:
             for name, n in self.ws_sizes.items():
@@ -272,7 +278,10 @@ class Plan:
             self._exec = _NativeOps([(_lib.OP_ZCONTRACT_WS, st.desc, st.refs + (("ws", "zc_work"),)) if wb else
                                      (_lib.OP_ZCONTRACT, st.desc, st.refs)
                                      for st, wb in zip(self.steps, self.work)])
-        self._exec.run(ws, x_ptr, y_ptr)
+        return self._exec
+
+    def run(self, x_ptr: int = 0, y_ptr: int = 0):
+        self.native_ops().run(self.ws, x_ptr, y_ptr)
 
 
 class ChainBuilder:
@@ -510,6 +519,11 @@ class MixedPlan:
             self._prep_exec = _NativeOps([(_lib.OP_TO_PLANES if kind == "conv" else _lib.OP_EXPAND_B, d,
                                            (refs[0], None, refs[1])) for kind, d, refs in self.prep])
 
+    def native_ops(self) -> "_NativeOps":
+        """The plan's launch list without the conversions of ``prep``."""
+        self._build_exec()
+        return self._exec
+
     def run(self, x_ptr: int = 0, y_ptr: int = 0):
         self._build_exec()
         if self.prep and not self.hold:
@@ -602,10 +616,17 @@ class KrylovSolver:
         first-order coupling (the adaptive stop then never triggers).
 
         ``apply(xp, yp)`` gets device pointers, or the basis row and the output
-        as tensors when it carries ``takes_tensors = True``. ``basis``, when
+        as tensors when it carries ``takes_tensors = True``; one that carries its
+        ``plan`` (a Plan or MixedPlan on this solver's workspace) is run from
+        native code for Hermitian operators (``_expm_plan``). ``basis``, when
         given, receives the Krylov basis (``Q``: m x n copy), the m x m
         projection used for the propagator (``T``) and the norm of x
         (``beta0``); the adjoint of the exponential reuses them."""
+        plan = getattr(apply, "plan", None)
+        # (an instrumented plan, one whose run() was replaced, keeps the loop below)
+        if plan is not None and hermitian and "run" not in vars(plan) and self.ws.device.type == "cuda":
+            return self._expm_plan(x, apply, plan, dt, exp_factor, krylov_tol, max_krylov_dim, out, tridiagonal,
+                                   basis)
         lib = _lib.load()
         stream = _stream_ptr()
         n = x.numel()
@@ -716,6 +737,79 @@ class KrylovSolver:
                 check(lib.ptn_zcombine(Q[i0:].data_ptr(), n, cnt, cdev[i0:].data_ptr(), tmp.data_ptr(), n,
                                        stream), "zcombine")
                 out.view(-1).add_(tmp)
+        return out
+
+
+    def _expm_plan(self, x, apply, plan, dt, exp_factor, krylov_tol, max_krylov_dim, out, tridiagonal, basis):
+        """``expm`` for an operator that is a plan: batches of steps and their
+        decisions in native code (``ptn_krylov_batch``), one synchronisation
+        per batch. The batches are those of ``expm``."""
+        lib = _lib.load()
+        stream = _stream_ptr()
+        ws = self.ws
+        n = x.numel()
+        out = x if out is None else out
+        if isinstance(plan, MixedPlan) and plan.prep and not plan.hold:
+            plan.prepare()
+        max_steps = n if max_krylov_dim is None else min(n, int(max_krylov_dim))
+        spec = self._spec_depth.get(n, 4) if n <= self.SPECULATE_MAX_N else 1
+        self._ensure_Q(x, n, min(max_steps + 1, max(spec + 1, 8)))
+        T = np.zeros((min(max_steps, 64) + 1,) * 2, dtype=complex)
+        d = _lib.KrylovDesc()
+        z = complex(exp_factor) * dt
+        d.x, d.n, d.tridiagonal, d.tol = x.data_ptr(), n, int(tridiagonal), float(krylov_tol)
+        d.z_re, d.z_im = z.real, z.imag
+        j = 0
+        while True:
+            batch = max(1, min(spec - j, max_steps - j)) if j < spec else 1
+            if j + batch + 1 > self._qcap:
+                self._ensure_Q(x, n, min(max_steps + 1, max(2 * self._qcap, j + batch + 1)))
+            batch = min(batch, self._qcap - j)
+            J = j + batch
+            if J + 1 > T.shape[0]:
+                T2 = np.zeros((max(2 * T.shape[0], J + 1),) * 2, dtype=complex)
+                T2[:T.shape[0], :T.shape[0]] = T
+                T = T2
+            coef = np.empty(J, dtype=complex)
+            hh, sc, st_host = self._pinned(J * (J + 1), 1 + 2 * J)
+            d.w = ws.get("kry_w", n).data_ptr()
+            d.h = ws.get("kry_hs", J * (J + 1)).data_ptr()
+            d.norms = ws.get("kry_sc", 1 + 2 * J, torch.float64).data_ptr()
+            d.partial = ws.get("kry_part", int(lib.ptn_krylov_partials(n)) + 8).data_ptr()
+            ops = plan.native_ops()
+            d.ptrs = ops.bind(ws)
+            d.ops, d.nops, d.nptrs = ops.ops, ops.n, len(ops.refs)
+            st = ws.bufs.get("tc_status")
+            d.status = st.data_ptr() if st is not None else None
+            d.Q, d.qcap = ws.ptr("kry_Q"), self._qcap
+            d.h_host, d.norms_host, d.status_host = hh.data_ptr(), sc.data_ptr(), st_host.data_ptr()
+            d.T, d.ldt, d.coef = T.ctypes.data, T.shape[0], coef.ctypes.data
+            d.j0, d.batch = j, batch
+            check(lib.ptn_krylov_batch(ctypes.byref(d), stream), "Krylov exponential")
+            if st is not None and int(st_host[0]) != 0:
+                code = int(st_host[0])
+                st.zero_()
+                raise _lib.PtnError(code, "tensor-core contraction inside the Krylov exponential")
+            j = J
+            if d.done or j >= max_steps:
+                break
+        m, beta0 = d.m, d.beta0
+        if beta0 == 0.0:
+            if out.data_ptr() != x.data_ptr():
+                out.copy_(x)
+            if basis is not None:
+                basis.update(Q=None, T=np.zeros((0, 0), dtype=complex), beta0=0.0, m=0)
+            return out
+        if n <= self.SPECULATE_MAX_N:
+            self._spec_depth[n] = m
+        self.depths.append(m)
+        ran = getattr(apply, "ran", None)
+        if ran is not None:
+            ran(j)                       # how often the operator was applied
+        if basis is not None:
+            Q = ws.bufs["kry_Q"][:m * n].view(m, n)
+            basis.update(Q=Q.clone(), T=self._proj(T, m, tridiagonal).copy(), beta0=beta0, m=m)
+        check(lib.ptn_krylov_combine(d.Q, n, m, d.coef, out.data_ptr(), stream), "krylov_combine")
         return out
 
 
@@ -987,16 +1081,24 @@ class DeviceNetwork:
         finally:
             p.hold = False
 
-    def evolve_site(self, nid, dt, exp_factor, tol, maxdim, hermitian: bool = True):
-        p = self.heff_plan(nid)
-
+    def _plan_apply(self, p):
+        """A plan as the operator of a local exponential."""
         def apply(xp, yp):
             p.run(xp, yp)
             self.flops += p.flops
+
+        def ran(count):
+            self.flops += p.flops * count
+        apply.plan, apply.ran = p, ran
+        return apply
+
+    def evolve_site(self, nid, dt, exp_factor, tol, maxdim, hermitian: bool = True):
+        p = self.heff_plan(nid)
         x = self.t[nid]
-        self._held(p, lambda: self.local_exp(x, apply, dt, exp_factor, tol, maxdim, hermitian, out=x))
+        self._held(p, lambda: self.local_exp(x, self._plan_apply(p), dt, exp_factor, tol, maxdim, hermitian, out=x))
         self._touch(nid)
-        self.check_device_status()
+        if self.ode is not None:         # the Krylov exponential reads the status word with its coefficients
+            self.check_device_status()
 
     def local_exp(self, x, apply, dt, exp_factor, tol, maxdim, hermitian=True, out=None):
         """exp(exp_factor dt H) x for the operator ``apply``: the Krylov
@@ -1019,11 +1121,7 @@ class DeviceNetwork:
 
     def evolve_bond(self, r: torch.Tensor, nid, nxt, dt, exp_factor, tol, maxdim, hermitian: bool = True):
         p = self.bond_plan(nid, nxt)
-
-        def apply(xp, yp):
-            p.run(xp, yp)
-            self.flops += p.flops
-        return self._held(p, lambda: self.local_exp(r, apply, dt, exp_factor, tol, maxdim, hermitian, out=r))
+        return self._held(p, lambda: self.local_exp(r, self._plan_apply(p), dt, exp_factor, tol, maxdim, hermitian, out=r))
 
     # -- QR split and R absorption ---------------------------------------------------
     # Reduced-precision path: tall splits (m >= 2k, k <= ptn_zchol_max_k) try
@@ -1640,12 +1738,9 @@ class DeviceNetwork:
         mp.run(0, x2.data_ptr())
         self.flops += mp.flops
         hp = self.heff2_plan(u, v)
-
-        def apply(xp, yp):
-            hp.run(xp, yp)
-            self.flops += hp.flops
-        self.local_exp(x2, apply, dt, exp_factor, tol, maxdim, hermitian, out=x2)
-        self.check_device_status()
+        self.local_exp(x2, self._plan_apply(hp), dt, exp_factor, tol, maxdim, hermitian, out=x2)
+        if self.ode is not None:
+            self.check_device_status()
         s = self.svd_split(u, v, x2, svd)
         self.state.orthogonality_center_id = v
         self.update_env(u, v)
