@@ -12,9 +12,12 @@
 //
 // The matrix is addressed in place inside the site tensor: element (i, c) at
 // A[rowoff[i] + c * colstride], where the row-offset table carries the
-// reference's (logical) row order. Each Householder step is a short sequence
-// of ordinary launches (column norm, reflector, column dots, dot reduction,
-// trailing update); no kernel waits on another.
+// reference's (logical) row order. Where the columns fit the chip's shared memory
+// the whole QR is one cooperative launch; a matrix of at most 2048 rows past that
+// takes one launch per reflector, a taller one a short sequence of launches (column
+// norm, reflector, column dots, dot reduction, trailing update).
+#include <type_traits>
+
 #include "ptn_common.cuh"
 
 namespace {
@@ -215,168 +218,251 @@ __global__ void zero_cols_kernel(double2* __restrict__ A, const int64_t* __restr
   }
 }
 
-// ---- small-m path: one launch per Householder step ------------------------------------
-// For m <= QR_SMALL_M each step is one kernel: every CTA recomputes the
-// reflector from column j (a few KB, identical arithmetic in every CTA, so the
-// result is the same everywhere) and then owns one trailing column (dot and
-// update). The reflectors go to a separate V buffer and the diagonal of R to
-// `betas`, so no CTA writes what another reads in the same launch.
+// ---- small m (at most QR_SMALL_M rows) --------------------------------------------------
+// Two forms of the same arithmetic: a launch sequence (one kernel per Householder
+// step) and, below, one cooperative launch. Both give the same bits: rows r, r +
+// HT, ... belong to thread r mod HT, a thread adds its rows in ascending order, the
+// lanes of a warp and then the four warps are added by a butterfly, and all
+// scalars come from the functions here. A reflector is kept unscaled: x = the
+// column below row j, s = 1 / (alpha - beta), v = (1, s x), so that
+//   v^H c = conj(s) x^H c + c_j,   H c = c - tau (v^H c) (1, s x),
+// which takes the scaling of v off the chain of dependent steps.
+//
+// What bounds a step on GB300 is the FP64 pipe and its latency: a warp
+// instruction holds a scheduler's FP64 unit for 64 cycles whatever the active
+// lanes. Hence four warps (one per scheduler) with several rows per thread, FMA
+// forms (4 per row and product), and sums of both parts of all of a CTA's columns
+// reduced together.
 constexpr int64_t QR_SMALL_M = 2048;
 constexpr int ST = 256;
+constexpr int HT = 128;                  // threads of the small-m kernels
+constexpr int HW = HT / 32;
 
-template <int NTH>
-__device__ __forceinline__ double block_sum(double v, double* red) {
-  v = warp_sum(v);
-  if (NTH == 32) return v;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) red[w] = v;
-  __syncthreads();
-  double s = 0.0;
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < NTH / 32; ++i) s += red[i];
-    red[NTH / 32] = s;
+// c - x g
+__device__ __forceinline__ double2 csub_mul(double2 c, double2 x, double2 g) {
+  c.x = fma(-x.x, g.x, c.x);
+  c.x = fma(x.y, g.y, c.x);
+  c.y = fma(-x.x, g.y, c.y);
+  c.y = fma(-x.y, g.x, c.y);
+  return c;
+}
+
+// zlarfg on (alpha, x) with |x|^2 = xn2: tau, s = 1 / (alpha - beta), beta and
+// nb = -1 / beta.
+struct Reflector {
+  double2 tau, s, beta;
+  double nb;
+};
+// Squared norms whose reciprocal may leave the range, and those that are not numbers.
+__device__ __noinline__ Reflector make_reflector_far(double2 alpha, double n2) {
+  Reflector h;
+  const double nrm = sqrt(n2), beta = alpha.x >= 0.0 ? -nrm : nrm;
+  h.beta = make_double2(beta, 0.0);
+  h.nb = -1.0 / beta;
+  h.tau = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
+  const double dx = alpha.x - beta, den = dx * dx + alpha.y * alpha.y;
+  h.s = make_double2(dx / den, -alpha.y / den);
+  return h;
+}
+__device__ __forceinline__ Reflector make_reflector(double2 alpha, double xn2) {
+  Reflector h;
+  if (xn2 == 0.0 && alpha.y == 0.0) {
+    h.tau = make_double2(0.0, 0.0);
+    h.s = make_double2(0.0, 0.0);
+    h.beta = alpha;
+    h.nb = 0.0;
+    return h;
   }
-  __syncthreads();
-  s = red[NTH / 32];
-  __syncthreads();
-  return s;
+  const double a2 = fma(alpha.x, alpha.x, alpha.y * alpha.y), n2 = a2 + xn2;
+  if (!(n2 > 1e-290 && n2 < 1e290)) return make_reflector_far(alpha, n2);
+  const bool pos = alpha.x >= 0.0;                   // beta = -sign(Re alpha) |(alpha, x)|
+  // one reciprocal square root for 1 / beta and, times n2, for beta itself with
+  // one correction; the reciprocal beside it does not wait for the correction
+  const double rn = rsqrt(n2), r0 = n2 * rn;
+  const double nrm = fma(fma(-r0, r0, n2), 0.5 * rn, r0);
+  const double rd = __drcp_rn(fma(2.0 * fabs(alpha.x), r0, a2 + n2));  // 1 / |alpha - beta|^2
+  h.beta = make_double2(pos ? -nrm : nrm, 0.0);
+  h.nb = pos ? rn : -rn;
+  h.tau = make_double2(fma(alpha.x, h.nb, 1.0), alpha.y * h.nb);  // (beta - alpha) / beta
+  h.s = make_double2((alpha.x - h.beta.x) * rd, -alpha.y * rd);
+  return h;
 }
 
-template <int NTH>
-__device__ __forceinline__ double2 block_sum2(double2 v, double* red) {
-  double re = block_sum<NTH>(v.x, red);
-  double im = block_sum<NTH>(v.y, red);
-  return make_double2(re, im);
-}
-
-// block_sum2 in one pass: both parts reduced with block_sum's tree (same warp
-// shuffles, warp partials added in warp order by thread 0), so the same bits,
-// with half the barriers. red2: NTH / 32 + 1 entries.
-template <int NTH>
-__device__ __forceinline__ double2 block_sum2_fused(double2 v, double2* red2) {
-  v.x = warp_sum(v.x);
-  v.y = warp_sum(v.y);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) red2[w] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double sx = 0.0, sy = 0.0;
-    for (int i = 0; i < NTH / 32; ++i) {
-      sx += red2[i].x;
-      sy += red2[i].y;
-    }
-    red2[NTH / 32] = make_double2(sx, sy);
+// f and g = s f of the update c_j - f, c_r - x_r g for a column with x^H c = d:
+// f = t (conj(s) d + c_j), t = conj(tau) in the factorisation and tau when Q is
+// formed. With conj(tau) conj(s) = tau s = nb one product is real. Even lanes form
+// the real parts, odd lanes the imaginary ones (five FP64 instructions instead
+// of twelve).
+template <bool FACTOR>
+__device__ __forceinline__ void reflect(double2 tau, double2 s, double nb, double2 d, double2 cj, double& f,
+                                        double& g) {
+  const bool im = threadIdx.x & 1;
+  const double dm = im ? d.y : d.x, cm = im ? cj.y : cj.x;
+  if (FACTOR) {
+    f = fma(tau.x, cm, fma(tau.y, im ? -cj.x : cj.y, nb * dm));
+    const double o = __shfl_xor_sync(0xffffffffu, f, 1);
+    g = fma(s.x, f, s.y * (im ? o : -o));
+  } else {
+    const double w = fma(s.x, dm, fma(s.y, im ? -d.x : d.y, cm));
+    const double o = __shfl_xor_sync(0xffffffffu, w, 1);
+    f = fma(tau.x, w, tau.y * (im ? o : -o));
+    g = nb * w;
   }
-  __syncthreads();
-  const double2 s = red2[NTH / 32];
-  __syncthreads();
-  return s;
+}
+__device__ __forceinline__ double2 pair_from(double v, int lane0) {
+  return make_double2(__shfl_sync(0xffffffffu, v, lane0), __shfl_sync(0xffffffffu, v, lane0 + 1));
 }
 
-// Step j of the factorisation. grid = max(1, k - j - 1); CTA b owns column j+1+b.
-template <int NTH>
-__global__ void __launch_bounds__(NTH) hh_fact_small(double2* __restrict__ A, const int64_t* __restrict__ rowoff,
+// CTA sums of 2 NC values (Re, Im of NC columns): partials in red[warp][value]
+// first, then, after the barrier, every lane gets value lane & (2 NC - 1)...
+// NC = 1 or 2.
+template <int NC>
+__device__ __forceinline__ void cta_partials(const double2 (&v)[NC], double (*red)[4]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (NC == 1) {
+    const bool up = lane & 16;
+    double t = (up ? v[0].y : v[0].x) + __shfl_xor_sync(0xffffffffu, up ? v[0].x : v[0].y, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if ((lane & 15) == 0) red[warp][lane >> 4] = t;
+  } else {
+    const bool up = lane & 16, hi = lane & 8;
+    const double2 keep = up ? v[NC - 1] : v[0], send = up ? v[0] : v[NC - 1];
+    const double a = keep.x + __shfl_xor_sync(0xffffffffu, send.x, 16);
+    const double b = keep.y + __shfl_xor_sync(0xffffffffu, send.y, 16);
+    double t = (hi ? b : a) + __shfl_xor_sync(0xffffffffu, hi ? a : b, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if ((lane & 7) == 0) red[warp][lane >> 3] = t;
+  }
+}
+template <int NC>
+__device__ __forceinline__ void cta_totals(double2 (&v)[NC], double (*red)[4]) {
+  // lane = warp index (2 bits) + 4 * value
+  const int lane = threadIdx.x & 31, val = (lane >> 2) & (2 * NC - 1);
+  double t = red[lane & 3][val];
+  t += __shfl_xor_sync(0xffffffffu, t, 1);
+  t += __shfl_xor_sync(0xffffffffu, t, 2);
+#pragma unroll
+  for (int i = 0; i < NC; ++i) {
+    v[i].x = __shfl_sync(0xffffffffu, t, 8 * i);
+    v[i].y = __shfl_sync(0xffffffffu, t, 8 * i + 4);
+  }
+}
+// one real value, the same tree
+__device__ __forceinline__ double cta_total1(double v, double (*red)[4]) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][0] = v;
+  __syncthreads();
+  double t = red[threadIdx.x & 3][0];
+  t += __shfl_xor_sync(0xffffffffu, t, 1);
+  t += __shfl_xor_sync(0xffffffffu, t, 2);
+  return __shfl_sync(0xffffffffu, t, 0);
+}
+
+// First row above j of this thread.
+__device__ __forceinline__ int64_t first_row(int64_t j) {
+  const int64_t r = (j + 1) / HT * HT + threadIdx.x;
+  return r > j ? r : r + HT;
+}
+
+// Step j of the factorisation. grid = max(1, k - j - 1); CTA b owns column j + 1 + b and
+// forms the reflector from column j itself (a few KB, the same bits in every
+// CTA). Reflectors go to V (unscaled) and tau / s, the diagonal of R to betas.
+__global__ void __launch_bounds__(HT) hh_fact_small(double2* __restrict__ A, const int64_t* __restrict__ rowoff,
                                                     int64_t cs, int64_t m, int64_t k, int64_t j,
-                                                    double2* __restrict__ tau, double2* __restrict__ betas,
-                                                    double2* __restrict__ V) {
-  __shared__ double2 vs[QR_SMALL_M];
-  __shared__ double red[NTH / 32 + 1];
-  __shared__ double2 sc[3];  // tau, scal, w
-  const int64_t len = m - j;
+                                                    double2* __restrict__ tau, double2* __restrict__ scal,
+                                                    double2* __restrict__ V, double2* __restrict__ R) {
+  __shared__ double red[2][HW][4];
+  const int tid = threadIdx.x;
   double acc = 0.0;
-  for (int64_t t = threadIdx.x; t < len; t += NTH) {
-    const double2 a = A[rowoff[j + t] + j * cs];
-    vs[t] = a;
-    if (t > 0) acc += cabs2(a);
+  for (int64_t r = first_row(j); r < m; r += HT) {
+    const double2 a = A[rowoff[r] + j * cs];
+    acc = fma(a.x, a.x, fma(a.y, a.y, acc));
+    if (blockIdx.x == 0) V[j * m + r] = a;
   }
-  const double xn2 = block_sum<NTH>(acc, red);
-  if (threadIdx.x == 0) {
-    const double2 alpha = vs[0];
-    const double xnorm = sqrt(xn2);
-    double2 t_, s_, b_;
-    if (xnorm == 0.0 && alpha.y == 0.0) {
-      t_ = make_double2(0.0, 0.0);
-      s_ = make_double2(0.0, 0.0);
-      b_ = alpha;
-    } else {
-      const double nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xnorm * xnorm);
-      const double beta = (alpha.x >= 0.0) ? -nrm : nrm;
-      t_ = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
-      const double2 d = make_double2(alpha.x - beta, alpha.y);
-      const double den = d.x * d.x + d.y * d.y;
-      s_ = make_double2(d.x / den, -d.y / den);
-      b_ = make_double2(beta, 0.0);
-    }
-    sc[0] = t_;
-    sc[1] = s_;
-    if (blockIdx.x == 0) {
-      tau[j] = t_;
-      betas[j] = b_;
-    }
+  const double xn2 = cta_total1(acc, red[0]);
+  const double2 alpha = A[rowoff[j] + j * cs];
+  const Reflector h = make_reflector(alpha, xn2);
+  if (blockIdx.x == 0 && tid == 0) {
+    tau[j] = h.tau;
+    scal[j] = h.s;
+    V[j * m + j] = make_double2(h.beta.x, h.nb);
+    R[j * k + j] = h.beta;
   }
-  __syncthreads();
-  const double2 s_ = sc[1];
-  for (int64_t t = threadIdx.x; t < len; t += NTH) {
-    const double2 v = (t == 0) ? make_double2(1.0, 0.0) : cmul(vs[t], s_);
-    vs[t] = v;
-    if (blockIdx.x == 0) V[j * m + j + t] = v;
-  }
-  __syncthreads();
   const int64_t c = j + 1 + blockIdx.x;
   if (c >= k) return;
-  double2 w = make_double2(0.0, 0.0);
-  for (int64_t t = threadIdx.x; t < len; t += NTH) w = cfmac(vs[t], A[rowoff[j + t] + c * cs], w);
-  w = block_sum2<NTH>(w, red);
-  double2 f = sc[0];
-  f.y = -f.y;  // conj(tau): the factorisation applies H^H
-  const double2 fw = cmul(f, w);
-  for (int64_t t = threadIdx.x; t < len; t += NTH) {
-    double2* p = A + rowoff[j + t] + c * cs;
-    *p = csub(*p, cmul(vs[t], fw));
+  double2 d[1] = {make_double2(0.0, 0.0)};
+  for (int64_t r = first_row(j); r < m; r += HT) d[0] = cfmac(A[rowoff[r] + j * cs], A[rowoff[r] + c * cs], d[0]);
+  cta_partials<1>(d, red[1]);
+  __syncthreads();
+  cta_totals<1>(d, red[1]);
+  double2* pj = A + rowoff[j] + c * cs;
+  const double2 cj = *pj;
+  __syncthreads();                                   // everyone has read c_j
+  double fl, gl;
+  reflect<true>(h.tau, h.s, h.nb, d[0], cj, fl, gl);
+  const double2 f = pair_from(fl, 0), g = pair_from(gl, 0);
+  if (tid == j % HT) *pj = csub(cj, f);
+  for (int64_t r = first_row(j); r < m; r += HT) {
+    double2* q = A + rowoff[r] + c * cs;
+    *q = csub_mul(*q, A[rowoff[r] + j * cs], g);
   }
 }
 
-// R[r][c]: strictly-upper part from A, diagonal from betas (rows < p), zero elsewhere.
+// R[r][c]: strictly-upper part from A (rows < p), zero elsewhere; the steps have
+// written the diagonal.
 __global__ void extract_r_small(const double2* __restrict__ A, const int64_t* __restrict__ rowoff, int64_t cs,
-                                int64_t k, int64_t p, const double2* __restrict__ betas, double2* __restrict__ R) {
+                                int64_t k, int64_t p, double2* __restrict__ R) {
   for (int64_t e = blockIdx.x * (int64_t)ST + threadIdx.x; e < k * k; e += (int64_t)gridDim.x * ST) {
     const int64_t r = e / k, c = e - r * k;
     double2 v = make_double2(0.0, 0.0);
-    if (r < p) {
-      if (c == r) v = betas[r];
-      else if (c > r) v = A[rowoff[r] + c * cs];
-    }
+    if (r < p && c == r) continue;
+    if (r < p && c > r) v = A[rowoff[r] + c * cs];
     R[e] = v;
   }
 }
 
+// Column c of H_c e_c: 1 - tau at row c, -(tau s) x = -nb x below.
+__device__ __forceinline__ double2 start_entry(int64_t r, int64_t c, double2 tau, double nb, double2 x) {
+  if (r < c) return make_double2(0.0, 0.0);
+  if (r == c) return make_double2(1.0 - tau.x, -tau.y);
+  return cscale(x, -nb);
+}
+
 // Step j of forming Q (zung2r): CTAs 0..ncols-1 apply H_j to columns j+1..p-1,
 // CTA ncols writes column j itself.
-template <int NTH>
-__global__ void __launch_bounds__(NTH) hh_form_small(double2* __restrict__ A, const int64_t* __restrict__ rowoff,
+__global__ void __launch_bounds__(HT) hh_form_small(double2* __restrict__ A, const int64_t* __restrict__ rowoff,
                                                     int64_t cs, int64_t m, int64_t p, int64_t j,
-                                                    const double2* __restrict__ tau, const double2* __restrict__ V) {
-  __shared__ double red[NTH / 32 + 1];
+                                                    const double2* __restrict__ tau,
+                                                    const double2* __restrict__ scal,
+                                                    const double2* __restrict__ V) {
+  __shared__ double red[HW][4];
   const int64_t ncols = p - (j + 1);
-  const double2 t_ = tau[j];
-  const double2* v = V + j * m;
+  const double2 t_ = tau[j], s_ = scal[j];
+  const double2* x = V + j * m;
   if (blockIdx.x == ncols) {
-    for (int64_t i = threadIdx.x; i < m; i += NTH) {
-      double2* q = A + rowoff[i] + j * cs;
-      if (i < j) *q = make_double2(0.0, 0.0);
-      else if (i == j) *q = make_double2(1.0 - t_.x, -t_.y);
-      else *q = make_double2(-(t_.x * v[i].x - t_.y * v[i].y), -(t_.x * v[i].y + t_.y * v[i].x));
-    }
+    for (int64_t r = threadIdx.x; r < m; r += HT)
+      A[rowoff[r] + j * cs] = start_entry(r, j, t_, x[j].y, r > j ? x[r] : make_double2(0.0, 0.0));
     return;
   }
   const int64_t c = j + 1 + blockIdx.x;
-  double2 w = make_double2(0.0, 0.0);
-  for (int64_t i = j + threadIdx.x; i < m; i += NTH) w = cfmac(v[i], A[rowoff[i] + c * cs], w);
-  w = block_sum2<NTH>(w, red);
-  const double2 fw = cmul(t_, w);
-  for (int64_t i = j + threadIdx.x; i < m; i += NTH) {
-    double2* q = A + rowoff[i] + c * cs;
-    *q = csub(*q, cmul(v[i], fw));
+  double2 d[1] = {make_double2(0.0, 0.0)};
+  for (int64_t r = first_row(j); r < m; r += HT) d[0] = cfmac(x[r], A[rowoff[r] + c * cs], d[0]);
+  cta_partials<1>(d, red);
+  __syncthreads();
+  cta_totals<1>(d, red);
+  double2* pj = A + rowoff[j] + c * cs;
+  const double2 cj = *pj;
+  __syncthreads();
+  double fl, gl;
+  reflect<false>(t_, s_, x[j].y, d[0], cj, fl, gl);
+  const double2 f = pair_from(fl, 0), g = pair_from(gl, 0);
+  if (threadIdx.x == j % HT) *pj = csub(cj, f);
+  for (int64_t r = first_row(j); r < m; r += HT) {
+    double2* q = A + rowoff[r] + c * cs;
+    *q = csub_mul(*q, x[r], g);
   }
 }
 
@@ -388,28 +474,33 @@ inline unsigned grid1(int64_t n) {
 }
 
 // ---- small m, one cooperative launch ---------------------------------------------------
-// The same Householder steps as hh_fact_small / extract_r_small / hh_form_small,
-// with the same arithmetic per column (thread-to-row map, reduction tree,
-// scalar formulas), so the results are the same bits; but all of them run in
-// one launch. CTA b owns a few columns (snake order, so the Q formation work
-// -- column c needs c + 1 reflectors -- is balanced) and keeps them in shared
-// memory. Reflector j is computed once, by the owner of column j, as soon as
-// column j has received reflectors 0 .. j-1, and published through V, tau and
-// a flag; every CTA waits for the flag (bounded), then applies the reflector
-// to its own columns. The owner of column j + 1 updates that column first and
-// publishes reflector j + 1 right away, so the chain of dependent steps costs
-// one flag hand-over each instead of one kernel launch.
+// CTA b owns a few columns (snake order, so the Q formation work -- column c needs
+// c + 1 reflectors -- is balanced) and keeps them in shared memory, each thread
+// its own rows. Reflector j is published by the owner of column j as soon as that
+// column has received reflectors 0 .. j-1: first the entries of x, each thread its
+// rows as it updates them, then, when the norm is known, tau and s. The buffers
+// start out filled with a NaN that no result can be, and readers poll the entries
+// they need: no flags and no fences, and the dot products with x run while the
+// owner still forms the scalars. The owner of column j + 1 updates that column
+// first. Chain per step: scalars - L2 - update - norm - scalars.
+// What bounds it is that chain (the arithmetic of 512 x 256 is 0.2 ms of the FP64
+// pipe): 4 us a step in the factorisation, of which norm, reflector and the two
+// barriers about 1.6, and 2.7 us a reflector when Q is formed. Two columns per CTA
+// rather than one: half as many readers of each x, one reduction for both.
+// Measured against flags with fences, 256 threads and scaled reflectors:
+// 512 x 256 3.28 -> 1.75 ms, 256 x 128 1.35 -> 0.64, 128 x 64 0.62 -> 0.28,
+// 16 x 8 0.086 -> 0.046, 2048 x 128 3.38 -> 2.66.
 constexpr long long HP_WAIT_CYCLES = 4000000000LL;   // ~2 s at 2 GHz
+constexpr unsigned long long HP_EMPTY = ~0ull;
 
 struct HPArgs {
   double2* A;
   const int64_t* rowoff;
   int64_t cs, m, k, p;
   double2* tau;
-  double2* betas;
+  double2* scal;
   double2* V;
   double2* R;
-  int* ready;     // [p], zero on entry; ready[j] = 1 once reflector j is published
   int* status;    // nonzero: a wait ran out (every CTA stops)
   int G;          // CTAs
   int cpc;        // columns per CTA (upper bound)
@@ -424,176 +515,254 @@ __device__ __forceinline__ int hp_owner(int64_t c, int G) {
   return (int)((i & 1) ? (G - 1 - r) : r);
 }
 
-__global__ void __launch_bounds__(ST) hh_persistent_kernel(HPArgs a) {
-  extern __shared__ double2 hsm[];           // [cpc][m] own columns, then [m] reflector
-  __shared__ double red[ST / 32 + 1];
-  __shared__ double2 red2[ST / 32 + 1];
-  __shared__ double2 sc[2];
-  __shared__ int abort_s;
+__device__ __forceinline__ void hp_put(double2* p, double2 v) {
+  // an input NaN may have any payload: not the empty one
+  unsigned long long a = (unsigned long long)__double_as_longlong(v.x), b = (unsigned long long)__double_as_longlong(v.y);
+  if (a == HP_EMPTY) a = 0x7ff8000000000000ull;
+  if (b == HP_EMPTY) b = 0x7ff8000000000000ull;
+  asm volatile("st.volatile.global.v2.u64 [%0], {%1,%2};" ::"l"(p), "l"(a), "l"(b) : "memory");
+}
+__device__ __forceinline__ bool hp_try(const double2* p, double2& v) {
+  unsigned long long a, b;
+  asm volatile("ld.volatile.global.v2.u64 {%0,%1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+  v = make_double2(__longlong_as_double((long long)a), __longlong_as_double((long long)b));
+  return a != HP_EMPTY && b != HP_EMPTY;
+}
+
+// This thread's rows below j of x_j, once published. False when the kernel must leave.
+template <int PF>
+__device__ __forceinline__ bool hp_wait_x(const HPArgs& a, int64_t j, double2 (&x)[PF]) {
+  const double2* v = a.V + j * a.m;
+  const long long t0 = clock64();
+  for (unsigned it = 1;; ++it) {
+    bool ok = true;
+#pragma unroll
+    for (int q = 0; q < PF; ++q) {
+      const int64_t r = threadIdx.x + (int64_t)q * HT;
+      x[q] = make_double2(0.0, 0.0);
+      if (r > j && r < a.m) ok = hp_try(v + r, x[q]) && ok;
+    }
+    if (__all_sync(0xffffffffu, ok)) return true;
+    int stop = 0;
+    if ((it & 255u) == 0u && *(volatile int*)a.status != 0) stop = 1;
+    if (clock64() - t0 > HP_WAIT_CYCLES) {
+      atomicExch(a.status, PTN_ERR_TIMEOUT);
+      stop = 1;
+    }
+    if (__any_sync(0xffffffffu, stop)) return false;
+  }
+}
+// tau, s and (beta, nb) of step j; `ready` says that they have been read already.
+__device__ __forceinline__ bool hp_try_scalars(const HPArgs& a, int64_t j, double2 (&sc)[3]) {
+  return hp_try(a.tau + j, sc[0]) & hp_try(a.scal + j, sc[1]) & hp_try(a.V + j * a.m + j, sc[2]);
+}
+__device__ __forceinline__ bool hp_wait_scalars(const HPArgs& a, int64_t j, double2 (&sc)[3], bool ready) {
+  const long long t0 = clock64();
+  for (unsigned it = 1;; ++it) {
+    const bool ok = ready || hp_try_scalars(a, j, sc);
+    if (__all_sync(0xffffffffu, ok)) return true;
+    ready = false;
+    int stop = 0;
+    if ((it & 255u) == 0u && *(volatile int*)a.status != 0) stop = 1;
+    if (clock64() - t0 > HP_WAIT_CYCLES) {
+      atomicExch(a.status, PTN_ERR_TIMEOUT);
+      stop = 1;
+    }
+    if (__any_sync(0xffffffffu, stop)) return false;
+  }
+}
+
+using Yes = std::true_type;
+using No = std::false_type;
+
+// PF: rows per thread (HT PF >= m).
+template <int PF>
+__global__ void __launch_bounds__(HT) hh_persistent_kernel(const HPArgs a) {
+  extern __shared__ double2 hsm[];           // [cpc][m] own columns
+  __shared__ double red[2][HW][4];
+  __shared__ double nred[HW][4];
+  __shared__ double2 head[2][2];             // c_j of the two columns in work
+  __shared__ int s_fail;
   const int b = blockIdx.x, tid = threadIdx.x, G = a.G;
   const int64_t m = a.m, k = a.k, p = a.p, cs = a.cs;
-  double2* vs = hsm + (int64_t)a.cpc * m;
   int nown = 0;
   while (nown < a.cpc && hp_col(b, nown, G) < k) ++nown;
   for (int i = 0; i < nown; ++i) {
     const int64_t c = hp_col(b, i, G);
-    for (int64_t t = tid; t < m; t += ST) hsm[i * m + t] = a.A[a.rowoff[t] + c * cs];
+    for (int64_t r = tid; r < m; r += HT) hsm[i * m + r] = a.A[a.rowoff[r] + c * cs];
   }
-  if (tid == 0) abort_s = 0;
+  if (tid == 0) s_fail = 0;
+  unsigned par = 0;                          // alternates the shared buffers of the sums
   __syncthreads();
 
-  // zlarfg on column j (own slot col) and publication of v_j, tau_j, beta_j
-  auto publish = [&](int64_t j, const double2* col) {
-    const int64_t len = m - j;
+  // norm, scalars and diagonal of column j (own slot col), whose entries are published
+  auto publish_scalars = [&](int64_t j, double2* col) {
     double acc = 0.0;
-    for (int64_t t = tid; t < len; t += ST)
-      if (t > 0) acc += cabs2(col[j + t]);
-    const double xn2 = block_sum<ST>(acc, red);
-    if (tid == 0) {
-      const double2 alpha = col[j];
-      const double xnorm = sqrt(xn2);
-      double2 t_, s_, b_;
-      if (xnorm == 0.0 && alpha.y == 0.0) {
-        t_ = make_double2(0.0, 0.0);
-        s_ = make_double2(0.0, 0.0);
-        b_ = alpha;
-      } else {
-        const double nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xnorm * xnorm);
-        const double beta = (alpha.x >= 0.0) ? -nrm : nrm;
-        t_ = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
-        const double2 d = make_double2(alpha.x - beta, alpha.y);
-        const double den = d.x * d.x + d.y * d.y;
-        s_ = make_double2(d.x / den, -d.y / den);
-        b_ = make_double2(beta, 0.0);
-      }
-      sc[1] = s_;
-      a.tau[j] = t_;
-      a.betas[j] = b_;
+#pragma unroll
+    for (int q = 0; q < PF; ++q) {
+      const int64_t r = tid + (int64_t)q * HT;
+      if (r > j && r < m) acc = fma(col[r].x, col[r].x, fma(col[r].y, col[r].y, acc));
     }
-    __syncthreads();
-    const double2 s_ = sc[1];
-    for (int64_t t = tid; t < len; t += ST)
-      a.V[j * m + j + t] = (t == 0) ? make_double2(1.0, 0.0) : cmul(col[j + t], s_);
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) atomicExch(a.ready + j, 1);
+    // the sum's barrier also makes alpha (thread j mod HT's row) visible
+    const double xn2 = cta_total1(acc, nred);
+    if (tid < 32) {
+      const Reflector h = make_reflector(col[j], xn2);
+      if (tid == 0) {
+        hp_put(a.tau + j, h.tau);
+        hp_put(a.scal + j, h.s);
+        hp_put(a.V + j * m + j, make_double2(h.beta.x, h.nb));
+        a.R[j * k + j] = h.beta;
+      }
+    }
+    __syncthreads();                         // nred is free again
+  };
+  auto publish_x = [&](int64_t j, const double2* col) {
+#pragma unroll
+    for (int q = 0; q < PF; ++q) {
+      const int64_t r = tid + (int64_t)q * HT;
+      if (r > j && r < m) hp_put(a.V + j * m + r, col[r]);
+    }
   };
 
-  if (p > 0 && hp_owner(0, G) == b) publish(0, hsm);      // column 0 is this CTA's slot 0
-  for (int64_t j = 0; j < p; ++j) {
-    if (tid == 0) {
-      const volatile int* flag = a.ready + j;
-      const volatile int* st = a.status;
-      const long long t0 = clock64();
-      for (unsigned it = 0;; ++it) {
-        if (*flag != 0) break;
-        if ((it & 255u) == 0u && *st != 0) { abort_s = 1; break; }
-        if (clock64() - t0 > HP_WAIT_CYCLES) {
-          atomicExch(a.status, PTN_ERR_TIMEOUT);
-          abort_s = 1;
-          break;
-        }
+  // one reflector on one or two own columns
+  auto apply = [&](auto factor, int64_t j, const double2 (&x)[PF], double2* c0, double2* c1, auto after) -> bool {
+    double2 sc[3];
+    const bool early = hp_try_scalars(a, j, sc);     // under way during the dot products
+    double2 d[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+#pragma unroll
+    for (int q = 0; q < PF; ++q) {
+      const int64_t r = tid + (int64_t)q * HT;
+      if (r > j && r < m) {
+        d[0] = cfmac(x[q], c0[r], d[0]);
+        if (c1) d[1] = cfmac(x[q], c1[r], d[1]);
       }
-      __threadfence();
+      if (r == j) {
+        head[par][0] = c0[r];
+        if (c1) head[par][1] = c1[r];
+      }
     }
+    cta_partials<2>(d, red[par]);
+    if (!hp_wait_scalars(a, j, sc, early)) s_fail = 1;
     __syncthreads();
-    if (abort_s) break;
-    const int64_t len = m - j;
-    // v_j and tau_j in one round trip to L2
-    if (tid == 0) sc[0] = __ldcg(a.tau + j);
-    for (int64_t t = tid; t < len; t += ST) vs[t] = __ldcg(a.V + j * m + j + t);
-    __syncthreads();
-    double2 f = sc[0];
-    f.y = -f.y;  // conj(tau): the factorisation applies H^H
-    for (int i = 0; i < nown; ++i) {
-      const int64_t c = hp_col(b, i, G);
-      if (c <= j) continue;
-      double2* col = hsm + i * m;
-      double2 w = make_double2(0.0, 0.0);
-      for (int64_t t = tid; t < len; t += ST) w = cfmac(vs[t], col[j + t], w);
-      w = block_sum2_fused<ST>(w, red2);
-      const double2 fw = cmul(f, w);
-      for (int64_t t = tid; t < len; t += ST) col[j + t] = csub(col[j + t], cmul(vs[t], fw));
-      __syncthreads();
-      if (c == j + 1 && j + 1 < p) publish(j + 1, col);
+    if (s_fail) return false;
+    cta_totals<2>(d, red[par]);
+    // lanes of the upper half work for the second column
+    const bool second = (tid & 16) != 0;
+    double f, g;
+    reflect<decltype(factor)::value>(sc[0], sc[1], sc[2].y, second ? d[1] : d[0], head[par][second ? 1 : 0], f, g);
+    const double2 f0 = pair_from(f, 0), g0 = pair_from(g, 0), f1 = pair_from(f, 16), g1 = pair_from(g, 16);
+#pragma unroll
+    for (int q = 0; q < PF; ++q) {
+      const int64_t r = tid + (int64_t)q * HT;
+      if (r > j && r < m) c0[r] = csub_mul(c0[r], x[q], g0);
+      if (r == j) c0[r] = csub(c0[r], f0);
     }
-    __syncthreads();
+    after();                                 // the first column is done
+    if (c1) {
+#pragma unroll
+      for (int q = 0; q < PF; ++q) {
+        const int64_t r = tid + (int64_t)q * HT;
+        if (r > j && r < m) c1[r] = csub_mul(c1[r], x[q], g1);
+        if (r == j) c1[r] = csub(c1[r], f1);
+      }
+    }
+    par ^= 1u;
+    return true;
+  };
+
+  double2 x[PF];
+  if (p > 0 && hp_owner(0, G) == b) {        // column 0 is this CTA's slot 0
+    publish_x(0, hsm);
+    publish_scalars(0, hsm);
   }
-  if (abort_s) {
-    if (b == 0 && tid == 0) a.R[0] = make_double2(NAN, NAN);   // the result is not usable
+  bool ok = true;
+  for (int64_t j = 0; j < p && ok; ++j) {
+    int i0 = 0;                              // own columns above j: slots i0 ..
+    while (i0 < nown && hp_col(b, i0, G) <= j) ++i0;
+    if (i0 == nown) break;
+    if (!hp_wait_x<PF>(a, j, x)) s_fail = 1; // seen by all at the next barrier
+    for (int i = i0; i < nown && ok; i += 2) {
+      double2* c0 = hsm + (int64_t)i * m;
+      const bool next = i == i0 && hp_col(b, i, G) == j + 1 && j + 1 < p;
+      ok = apply(Yes{}, j, x, c0, i + 1 < nown ? c0 + m : nullptr, [&]() {
+        if (next) {
+          publish_x(j + 1, c0);
+          publish_scalars(j + 1, c0);
+        }
+      });
+    }
+  }
+  if (!ok) {
+    if (tid == 0) a.R[0] = make_double2(NAN, NAN);   // the result is not usable
     return;
   }
-  // R (rows < p: beta on the diagonal, the stored upper part above it), then Q
-  // (zung2r: column c = H_0 ... H_c e_c), KEEP padding past p
+  __syncthreads();
+  // R above the diagonal and its zeros (rows < p: the diagonal is written with the
+  // scalars), then Q (zung2r: column c = H_0 ... H_c e_c), KEEP padding past p
   for (int i = 0; i < nown; ++i) {
     const int64_t c = hp_col(b, i, G);
-    double2* col = hsm + i * m;
-    for (int64_t r = tid; r < k; r += ST) {
-      double2 v = make_double2(0.0, 0.0);
-      if (r < p) {
-        if (c == r) v = a.betas[r];
-        else if (c > r) v = col[r];
-      }
-      a.R[r * k + c] = v;
+    const double2* col = hsm + (int64_t)i * m;
+    for (int64_t r = tid; r < k; r += HT)
+      if (!(r == c && r < p)) a.R[r * k + c] = (r < p && c > r) ? col[r] : make_double2(0.0, 0.0);
+  }
+  // column c starts from its own reflector, still in its slot
+  for (int i = 0; i < nown; ++i) {
+    const int64_t c = hp_col(b, i, G);
+    double2* col = hsm + (int64_t)i * m;
+    if (c < p) {
+      double2 sc[3];
+      if (!hp_wait_scalars(a, c, sc, false)) s_fail = 1;
+      for (int64_t r = tid; r < m; r += HT) col[r] = start_entry(r, c, sc[0], sc[2].y, col[r]);
+    } else {
+      for (int64_t r = tid; r < m; r += HT) col[r] = make_double2(0.0, 0.0);
     }
-    __syncthreads();
-    if (c >= p) {
-      for (int64_t t = tid; t < m; t += ST) a.A[a.rowoff[t] + c * cs] = make_double2(0.0, 0.0);
-      continue;
-    }
-    // reflectors come from other CTAs: read them through L2
-    const double2 tc = __ldcg(a.tau + c);
-    const double2* vc = a.V + c * m;
-    for (int64_t t = tid; t < m; t += ST) {
-      if (t < c) {
-        col[t] = make_double2(0.0, 0.0);
-      } else if (t == c) {
-        col[t] = make_double2(1.0 - tc.x, -tc.y);
-      } else {
-        const double2 vt = __ldcg(vc + t);
-        col[t] = make_double2(-(tc.x * vt.x - tc.y * vt.y), -(tc.x * vt.y + tc.y * vt.x));
-      }
-    }
-    __syncthreads();
-    // H_{c-1}, ..., H_0 in turn; each step stages its reflector in shared
-    // memory, and the next one is fetched while this one is applied
-    constexpr int PF = QR_SMALL_M / ST;                // rows per thread
-    double2 pre[PF];
-    double2 tpre = make_double2(0.0, 0.0);
-    if (c > 0) {
-      const double2* v = a.V + (c - 1) * m;
+  }
+  __syncthreads();
+  ok = s_fail == 0;
+  __syncthreads();
+  // reflectors from the highest column down, on pairs of own columns (the later
+  // column of a pair alone until the earlier one's turn comes); each x is
+  // fetched while the one before it is applied
+  for (int i = 0; i < nown && ok; i += 2) {
+    const int64_t ca = hp_col(b, i, G), cb = i + 1 < nown ? hp_col(b, i + 1, G) : -1;
+    double2* pa = hsm + (int64_t)i * m;
+    double2* pb = pa + m;
+    const int64_t la = ca < p ? ca : 0, lb = cb >= 0 && cb < p ? cb : 0;   // reflectors still to apply
+    double2 nx[PF];
+    const int64_t top = la > lb ? la : lb;
+    if (top > 0 && !hp_wait_x<PF>(a, top - 1, nx)) s_fail = 1;
+    for (int64_t j = top - 1; j >= 0 && ok; --j) {
 #pragma unroll
-      for (int q = 0; q < PF; ++q) {
-        const int64_t t = (c - 1) + tid + (int64_t)q * ST;
-        pre[q] = t < m ? __ldcg(v + t) : make_double2(0.0, 0.0);
-      }
-      tpre = __ldcg(a.tau + (c - 1));
-    }
-    for (int64_t j = c - 1; j >= 0; --j) {
-#pragma unroll
-      for (int q = 0; q < PF; ++q) {
-        const int64_t t = j + tid + (int64_t)q * ST;
-        if (t < m) vs[t] = pre[q];
-      }
-      const double2 t_ = tpre;
+      for (int q = 0; q < PF; ++q) x[q] = nx[q];
       if (j > 0) {
-        const double2* vn = a.V + (j - 1) * m;
+        const double2* v = a.V + (j - 1) * m;        // published long ago
 #pragma unroll
         for (int q = 0; q < PF; ++q) {
-          const int64_t t = (j - 1) + tid + (int64_t)q * ST;
-          pre[q] = t < m ? __ldcg(vn + t) : make_double2(0.0, 0.0);
+          const int64_t r = tid + (int64_t)q * HT;
+          nx[q] = (r >= j && r < m) ? __ldcg(v + r) : make_double2(0.0, 0.0);
         }
-        tpre = __ldcg(a.tau + (j - 1));
       }
-      double2 w = make_double2(0.0, 0.0);
-      for (int64_t t = j + tid; t < m; t += ST) w = cfmac(vs[t], col[t], w);
-      w = block_sum2_fused<ST>(w, red2);
-      const double2 fw = cmul(t_, w);
-      for (int64_t t = j + tid; t < m; t += ST) col[t] = csub(col[t], cmul(vs[t], fw));
-      __syncthreads();
+      if (j < la) ok = apply(No{}, j, x, pa, j < lb ? pb : nullptr, []() {});
+      else ok = apply(No{}, j, x, pb, nullptr, []() {});
     }
-    for (int64_t t = tid; t < m; t += ST) a.A[a.rowoff[t] + c * cs] = col[t];
   }
+  if (!ok) {
+    if (tid == 0) a.R[0] = make_double2(NAN, NAN);
+    return;
+  }
+  for (int i = 0; i < nown; ++i) {
+    const int64_t c = hp_col(b, i, G);
+    for (int64_t r = tid; r < m; r += HT) a.A[a.rowoff[r] + c * cs] = hsm[(int64_t)i * m + r];
+  }
+}
+
+const void* hp_kernel(int64_t m) {
+  const int64_t pf = (m + HT - 1) / HT;
+  if (pf <= 1) return (const void*)hh_persistent_kernel<1>;
+  if (pf <= 2) return (const void*)hh_persistent_kernel<2>;
+  if (pf <= 4) return (const void*)hh_persistent_kernel<4>;
+  if (pf <= 8) return (const void*)hh_persistent_kernel<8>;
+  return (const void*)hh_persistent_kernel<16>;
 }
 
 }  // namespace
@@ -601,7 +770,7 @@ __global__ void __launch_bounds__(ST) hh_persistent_kernel(HPArgs a) {
 extern "C" int64_t ptn_zqr_work_bytes(int64_t m, int64_t k) {
   if (m <= QR_SMALL_M) {
     const int64_t p = m < k ? m : k;
-    return 16 * (2 * k + m * p) + 4 * (p + 1) + 512;   // tau, betas, V, flags, status
+    return 16 * (2 * k + m * p) + 4 * (p + 1) + 512;   // tau, s, V, status
   }
   return 16 * (3 * k + (nrb_for(m) + 1) / 2 + 1 + nrb_for(m) * k) + 256;
 }
@@ -624,9 +793,9 @@ static bool hp_shape(int64_t m, int64_t k, int& G, int& cpc, size_t& smem) {
         !pr.cooperativeLaunch)
       return d;
     const size_t dyn = pr.sharedMemPerBlockOptin - 1024;    // room for the static shared memory
-    if (cudaFuncSetAttribute(hh_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn) !=
-        cudaSuccess)
-      return d;
+    for (int64_t rows = HT; rows <= QR_SMALL_M; rows *= 2)
+      if (cudaFuncSetAttribute(hp_kernel(rows), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn) != cudaSuccess)
+        return d;
     d.n_sm = pr.multiProcessorCount;
     d.dyn_max = dyn;
     return d;
@@ -635,10 +804,10 @@ static bool hp_shape(int64_t m, int64_t k, int& G, int& cpc, size_t& smem) {
   int64_t g = (k + 1) / 2;                           // two columns per CTA
   if (g > dv.n_sm) g = dv.n_sm;
   const int64_t c = (k + g - 1) / g;
-  const size_t bytes = (size_t)(c + 1) * (size_t)m * sizeof(double2);
+  const size_t bytes = (size_t)c * (size_t)m * sizeof(double2);
   if (bytes > dv.dyn_max) return false;
   int max_per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&max_per_sm, hh_persistent_kernel, ST, bytes) != cudaSuccess ||
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&max_per_sm, hp_kernel(m), HT, bytes) != cudaSuccess ||
       (int64_t)max_per_sm * dv.n_sm < g)
     return false;
   G = (int)g;
@@ -668,18 +837,19 @@ static int zqr_keep_persistent(double2* A, const int64_t* rowoff, int64_t m, int
   a.k = k;
   a.p = p;
   a.tau = static_cast<double2*>(work);
-  a.betas = a.tau + k;
-  a.V = a.betas + k;
-  a.ready = reinterpret_cast<int*>(a.V + m * p);
-  a.status = a.ready + p;
+  a.scal = a.tau + k;
+  a.V = a.scal + k;
+  a.status = reinterpret_cast<int*>(a.V + m * p);
   a.R = R;
   a.G = G;
   a.cpc = cpc;
-  if (cudaMemsetAsync(a.ready, 0, sizeof(int) * (size_t)(p + 1), s) != cudaSuccess) return PTN_ERR_LAUNCH;
+  // every entry empty
+  if (cudaMemsetAsync(a.tau, 0xff, sizeof(double2) * (size_t)(2 * k + m * p), s) != cudaSuccess ||
+      cudaMemsetAsync(a.status, 0, sizeof(int), s) != cudaSuccess)
+    return PTN_ERR_LAUNCH;
   void* args[] = {&a};
   PTN_COUNT(1);
-  if (cudaLaunchCooperativeKernel((const void*)hh_persistent_kernel, dim3((unsigned)G), dim3(ST), args, smem, s) !=
-      cudaSuccess)
+  if (cudaLaunchCooperativeKernel(hp_kernel(m), dim3((unsigned)G), dim3(HT), args, smem, s) != cudaSuccess)
     return PTN_ERR_LAUNCH;
   return ptn_launch_status();
 }
@@ -687,20 +857,19 @@ static int zqr_keep_persistent(double2* A, const int64_t* rowoff, int64_t m, int
 static int zqr_keep_small(double2* A, const int64_t* rowoff, int64_t m, int64_t k, int64_t cs, double2* R,
                           void* work, cudaStream_t s) {
   double2* tau = static_cast<double2*>(work);
-  double2* betas = tau + k;
-  double2* V = betas + k;
+  double2* scal = tau + k;
+  double2* V = scal + k;
   const int64_t p = m < k ? m : k;
-  // (one warp per column measured slower than 256 threads at 512 x 256: 6.8 vs 4.2 ms)
   for (int64_t j = 0; j < p; ++j) {
     const int64_t ncols = k - (j + 1);
     PTN_COUNT(1);
-    hh_fact_small<ST><<<(unsigned)(ncols > 0 ? ncols : 1), ST, 0, s>>>(A, rowoff, cs, m, k, j, tau, betas, V);
+    hh_fact_small<<<(unsigned)(ncols > 0 ? ncols : 1), HT, 0, s>>>(A, rowoff, cs, m, k, j, tau, scal, V, R);
   }
   PTN_COUNT(1);
-  extract_r_small<<<grid1(k * k), ST, 0, s>>>(A, rowoff, cs, k, p, betas, R);
+  extract_r_small<<<grid1(k * k), ST, 0, s>>>(A, rowoff, cs, k, p, R);
   for (int64_t j = p - 1; j >= 0; --j) {
     PTN_COUNT(1);
-    hh_form_small<ST><<<(unsigned)(p - j), ST, 0, s>>>(A, rowoff, cs, m, p, j, tau, V);
+    hh_form_small<<<(unsigned)(p - j), HT, 0, s>>>(A, rowoff, cs, m, p, j, tau, scal, V);
   }
   if (p < k) { PTN_COUNT(1); zero_cols_kernel<<<grid1(m * (k - p)), QT, 0, s>>>(A, rowoff, cs, m, k, p); }
   return ptn_launch_status();
