@@ -169,7 +169,7 @@ int ptn_znonzero_rows(const void* A, const int64_t* rowoff, int64_t m, int64_t k
  *
  * G (k x k, row-major, leading dimension ldg, Hermitian up to rounding; its
  * Hermitian part is used) = R^H R with R upper triangular: writes R and R^{-1}
- * (k x k row-major, zero below the diagonal). Computed in FP32 on one CTA.
+ * (k x k row-major, zero below the diagonal). Computed in FP32 on one cluster.
  * status (device int32) is set to PTN_ERR_NOCONVERGE when a pivot is not
  * positive or the smallest diagonal entry of R is not above pivot_ratio times
  * the largest (the matrix is not of full numerical rank; the caller falls back
