@@ -7,7 +7,8 @@
 //   L = 3 ("BF16x6"): + A0B2 + A1B1 + A2B0, relative error ~2^-24 (FP32 level).
 // The complex product is written as one real product with doubled width:
 //   [Cr | Ci] = Ar * [Br | Bi] + Ai * [-Bi | Br]
-// so each (i, j) term issues two tcgen05.mma (M=128, N=2*NT, K=16). The
+// so each (i, j) term issues two tcgen05.mma (M=128, N=2*NT, K=16; NT = 64 or 128
+// complex columns). The
 // expanded B keeps the three blocks [-Bi; Br; Bi] of a level adjacent in shared
 // memory, so the Ar operand is the window [Br; Bi] and the Ai operand the
 // window [-Bi; Br].
@@ -17,9 +18,11 @@
 //   Bx: bf16 [level][block(-Bi, Br, Bi)][N][ldb]
 // Tiles are staged by TMA (32-byte swizzle, K=16 per stage, up to 8 stages)
 // through an mbarrier ring; two stages make one 32-wide accumulation round;
-// one warp issues TMA, one warp issues MMA and owns the TMEM allocation, four
-// warps run the epilogue (TMEM -> registers -> global, strided by output mode
-// tables so the result lands directly in the layout the next step reads).
+// one warp issues TMA, one warp issues MMA and owns the TMEM allocation, four or
+// eight warps run the epilogue (TMEM -> registers -> global, strided by output mode
+// tables so the result lands directly in the layout the next step reads). A CTA
+// stays on its SM and goes from tile to tile: while its epilogue writes one tile,
+// loads and MMAs of the next run on.
 // Every mbarrier wait is bounded; a timeout sets *status and the CTA exits.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -31,25 +34,27 @@
 namespace {
 
 constexpr int MT = 128;         // rows of C per CTA
-constexpr int NT = 64;          // complex columns of C per CTA (MMA N = 2*NT)
 constexpr int KT = 32;          // K per accumulation round (the unit of the K split)
 constexpr int KS = 16;          // K per shared-memory stage (one 32-byte swizzle row, one MMA K)
 constexpr int A_PLANE_BYTES = MT * 2 * KS;         // 4 KB
-constexpr int B_BLOCK_BYTES = NT * 2 * KS;         // 2 KB
 constexpr int SMEM_LIMIT = 227 * 1024;
-constexpr int THREADS = 192;
+constexpr int TMEM_COLS = 512;
+constexpr int EC = 64;          // complex columns of an epilogue thread's row
 
 // Stages of KS: as many as fit (at most 8). Two stages make one accumulation
-// round, so the TMEM partial sums still cover 32 K values; the deeper ring
-// hides the TMA latency that two 84 KB stages of 32 K values left exposed
-// (ncu at the chi=128 root: tensor pipe 39 % active, long-scoreboard stalls).
-template <int L>
+// round, so the TMEM partial sums cover 32 K values.
+// NT: complex columns of C per CTA (MMA N = 2*NT).
+template <int L, int NT>
 struct Cfg {
+  static constexpr int B_BLOCK = NT * 2 * KS;
   static constexpr int A_STAGE = 2 * L * A_PLANE_BYTES;
-  static constexpr int B_STAGE = 3 * L * B_BLOCK_BYTES;
+  static constexpr int B_STAGE = 3 * L * B_BLOCK;
   static constexpr int STAGE = A_STAGE + B_STAGE;
-  static constexpr int STAGES = (SMEM_LIMIT - 2048) / STAGE > 8 ? 8 : (SMEM_LIMIT - 2048) / STAGE;
+  static constexpr int STAGES = (SMEM_LIMIT - 4096) / STAGE > 8 ? 8 : (SMEM_LIMIT - 4096) / STAGE;
   static constexpr int SMEM = STAGES * STAGE + 1024;
+  static constexpr int EPI_WARPS = 4 * (NT / EC);
+  static constexpr int THREADS = 64 + 32 * EPI_WARPS;
+  static constexpr int NBUF = TMEM_COLS / (2 * NT);   // TMEM accumulators
 };
 constexpr long long WAIT_CYCLES = 4000000000LL;    // ~2 s at 2 GHz
 
@@ -66,12 +71,25 @@ struct GemmArgs {
   int64_t c_plane;           // plane stride (elements) for out_kind 1
   OutModes mo, no;
   int32_t* status;
-  int64_t tiles_n;
-  int64_t tiles;             // output tiles (tiles_m * tiles_n)
+  int32_t tiles_m;           // row blocks of C
+  int32_t items;             // tiles times K ranges
   int32_t splits;            // K ranges per tile (1: no split)
-  int32_t ksplit;            // K tiles per range
+  int32_t ksplit;            // K tiles (KT) per range
   float2* partial;           // [splits][M][N] FP32 partial sums when splits > 1
+  int32_t store;             // how the epilogue writes (StoreKind)
 };
+
+// Stores of the epilogue, where a thread holds 64 columns of one row. Single entries
+// of BF16 planes whose columns are the contiguous index are 2-byte pieces of 32
+// sectors an instruction, 50 us for one 128 x 64 tile; hence
+//   ROW8, 4, 2: that many columns of a row together (innermost column mode of stride 1);
+//   PAIR4, 2: that many columns of two rows (innermost row mode of stride 1 and even
+//         extent, innermost column mode of stride 2: a site's physical leg of
+//         dimension 2), neighbour lanes exchange halves;
+//   PAIR: one column of two rows (the same row mode, any column modes).
+// Every other stride, the plane stride and the base are then multiples of a store
+// (store_kind). Complex128 (ROW2) and partial sums (ROW4) go out 32 bytes at a time.
+enum StoreKind { ST_ONE = 0, ST_ROW8, ST_ROW4, ST_ROW2, ST_PAIR4, ST_PAIR2, ST_PAIR };
 
 // Split-K: outputs with fewer tiles than this many CTAs get their K range
 // split so the launch fills the GPU (one CTA per SM, 152 SMs, two waves);
@@ -93,57 +111,180 @@ __device__ __forceinline__ int64_t decode_off(const OutModes& md, int64_t idx) {
   return o;
 }
 
-template <int L>
-__global__ void __launch_bounds__(THREADS, 1)
+// The same for an index and extents below 2^31.
+__device__ __forceinline__ int64_t decode_off32(const OutModes& md, uint32_t idx) {
+  int64_t o = 0;
+  for (int d = md.n - 1; d >= 0; --d) {
+    const uint32_t dim = (uint32_t)md.dim[d], q = idx / dim;
+    o += (int64_t)(idx - q * dim) * md.stride[d];
+    idx = q;
+  }
+  return o;
+}
+
+// Work items (K range, tile): CTA b takes b, b + gridDim.x, ... Tiles of a row block of
+// C follow one another, so that CTAs which run together share A in L2; the narrow tiles
+// that a ragged N leaves come last, where they even out the CTAs' shares.
+struct Item {
+  int64_t m0, n0;
+  int split, k0, stages;         // first stage and stages of KS of the K range
+};
+template <int NT>
+__device__ __forceinline__ Item item_at(const GemmArgs& g, uint32_t w) {
+  Item it;
+  const uint32_t full = (uint32_t)(g.N / NT), tm_all = (uint32_t)g.tiles_m;
+  const uint32_t whole = full * tm_all * (uint32_t)g.splits;
+  uint32_t tm;
+  if (w < whole) {
+    const uint32_t r = w / full;
+    it.n0 = (int64_t)(w - r * full) * NT;
+    it.split = (int)(r / tm_all);
+    tm = r - (uint32_t)it.split * tm_all;
+  } else {
+    w -= whole;
+    it.n0 = (int64_t)full * NT;
+    it.split = (int)(w / tm_all);
+    tm = w - (uint32_t)it.split * tm_all;
+  }
+  it.m0 = (int64_t)tm * MT;
+  const int all = (int)((g.K + KS - 1) / KS), per = g.ksplit * (KT / KS);
+  it.k0 = it.split * per;        // the ranges are whole accumulation rounds (KT)
+  it.stages = min(all, it.k0 + per) - it.k0;
+  return it;
+}
+
+__device__ __forceinline__ void st_global_32(void* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e,
+                                             uint32_t f, uint32_t g, uint32_t h) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d), "r"(e),
+               "r"(f), "r"(g), "r"(h)
+               : "memory");
+}
+
+// v = bf16(x); x -= v
+__device__ __forceinline__ uint32_t take_bf16(float& x) {
+  const __nv_bfloat16 b = __float2bfloat16_rn(x);
+  x -= __bfloat162float(b);
+  return (uint32_t)__bfloat16_as_ushort(b);
+}
+
+__device__ __forceinline__ void put_words(__nv_bfloat16* p, const uint32_t* w, int n) {
+  if (n == 4) *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+  else if (n == 2) *reinterpret_cast<uint2*>(p) = make_uint2(w[0], w[1]);
+  else *reinterpret_cast<uint32_t*>(p) = w[0];
+}
+
+// Eight columns of one plane, x[0..7] (their next BF16 piece), from a lane's row.
+// no: the offsets of the eight columns (-1: past the end). Whole warps come here:
+// lanes exchange.
+template <int KIND>
+__device__ __forceinline__ void store_plane8(__nv_bfloat16* __restrict__ C, float* x, const int64_t* no, bool row_ok) {
+  constexpr bool ROW = KIND == ST_ROW8 || KIND == ST_ROW4 || KIND == ST_ROW2;
+  constexpr bool QUAD = KIND == ST_PAIR4 || KIND == ST_PAIR2;
+  uint32_t v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = take_bf16(x[i]);
+  const bool odd = threadIdx.x & 1;
+  if (KIND == ST_ONE || ((ROW || QUAD) && no[7] < 0)) {      // or the last columns
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (row_ok && no[i] >= 0) C[no[i]] = __ushort_as_bfloat16((unsigned short)v[i]);
+  } else if constexpr (ROW) {
+    constexpr int V = KIND == ST_ROW8 ? 8 : (KIND == ST_ROW4 ? 4 : 2);
+    const uint32_t w[4] = {v[0] | v[1] << 16, v[2] | v[3] << 16, v[4] | v[5] << 16, v[6] | v[7] << 16};
+    if (row_ok) {
+#pragma unroll
+      for (int i = 0; i < 8; i += V) put_words(C + no[i], w + i / 2, V / 2);
+    }
+  } else if constexpr (QUAD) {
+    // of 2 V columns the even lane writes the first V of both rows, the odd one the last
+    constexpr int V = KIND == ST_PAIR4 ? 4 : 2;
+#pragma unroll
+    for (int g = 0; g < 8; g += 2 * V) {
+      uint32_t w[V];
+#pragma unroll
+      for (int i = 0; i < V; i += 2) {
+        const uint32_t mine = odd ? (v[g + i] | v[g + i + 1] << 16) : (v[g + V + i] | v[g + V + i + 1] << 16);
+        const uint32_t r = __shfl_xor_sync(0xffffffffu, mine, 1);
+        w[i] = odd ? ((r & 0xffffu) | v[g + V + i] << 16) : (v[g + i] | r << 16);
+        w[i + 1] = odd ? (r >> 16 | v[g + V + i + 1] << 16) : (v[g + i + 1] | (r & 0xffff0000u));
+      }
+      if (row_ok) put_words(C + (odd ? no[g + V] - 1 : no[g]), w, V);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+      const uint32_t r = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 1);
+      const int64_t n = odd ? no[i + 1] : no[i];
+      if (row_ok && n >= 0)
+        *reinterpret_cast<uint32_t*>(C + n - (odd ? 1 : 0)) = odd ? (r | v[i + 1] << 16) : (v[i] | r << 16);
+    }
+  }
+}
+template <int L, int KIND>
+__device__ __forceinline__ void store_planes(__nv_bfloat16* __restrict__ C, int64_t ps, float (&re)[EC],
+                                             float (&im)[EC], const int64_t* no, bool row_ok) {
+#pragma unroll
+  for (int i = 0; i < EC; i += 8) {
+    if (no[i] < 0) break;                   // the same in all lanes
+#pragma unroll
+    for (int lv = 0; lv < L; ++lv) {
+      store_plane8<KIND>(C + (2 * lv) * ps, re + i, no + i, row_ok);
+      store_plane8<KIND>(C + (2 * lv + 1) * ps, im + i, no + i, row_ok);
+    }
+  }
+}
+
+// What bounds it: the tensor pipe against shared memory. An MMA of N = 128 takes 64
+// cycles and reads 8 KB of operands, all that shared memory gives, and the stages
+// have to be written too; one of N = 256 reads 12 KB in 128 cycles. And every tile
+// pays for its start (barriers, TMEM, tensor maps, first loads) and its output,
+// 25 us of a K = 1280 tile's 65 and 13 of a K = 256 tile's 20 when a CTA did one tile
+// each. Hence NT = 128 where there are tiles enough (launch_gemm), and persistent
+// CTAs: two accumulation rounds of the next tile fit in TMEM while the epilogue
+// writes. Measured (BF16x6, tensor-pipe rate counts the six products):
+// 655360 x 256 x 1280 8.65 -> 6.86 ms (1190 -> 1500 TFLOP/s), 131072 x 1280 x 256 into
+// rows of ten 3.11 -> 1.70, 131072 x 256 x 256 into complex128 0.54 -> 0.34, 40000 x 200
+// x 136 into planes by rows 0.51 -> 0.14, 640 x 128 x 640 into pairs 67 -> 47 us.
+template <int L, int NT>
+__global__ void __launch_bounds__(64 + 128 * (NT / EC), 1)
     cgemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const GemmArgs g) {
-  using C_ = Cfg<L>;
+  using C_ = Cfg<L, NT>;
   constexpr int STAGES = C_::STAGES;
   constexpr int STAGE_BYTES = C_::STAGE;
   constexpr int A_STAGE_BYTES = C_::A_STAGE;
+  constexpr int B_BLOCK_BYTES = C_::B_BLOCK;
+  constexpr int NBUF = C_::NBUF;
   constexpr uint32_t ACC_COLS = 2 * NT;          // one accumulator: [Re | Im]
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], tfull_bar[2], tempty_bar[2], drain_bar;
+  __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], tfull_bar[NBUF], tempty_bar[NBUF], drain_bar;
   __shared__ uint32_t tmem_base;
-  __shared__ int64_t noff[NT];
+  __shared__ int64_t noff_s[C_::EPI_WARPS][EC];
   __shared__ int s_abort;
   const volatile int32_t* vstatus = g.status;
   if (threadIdx.x == 0) s_abort = *vstatus;
   __syncthreads();
-  if (s_abort != 0) return;  // an earlier CTA failed: skip the work
+  if (s_abort != 0) return;  // an earlier launch failed: skip the work
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t tile = blockIdx.x % g.tiles;
-  const int split = (int)(blockIdx.x / g.tiles);
-  const int64_t tm = tile / g.tiles_n, tn = tile - tm * g.tiles_n;
-  const int64_t m0 = tm * MT, n0 = tn * NT;
-  // stages of KS K values; the split ranges are whole accumulation rounds (KT)
-  const int kt_all = (int)((g.K + KS - 1) / KS);
-  const int kt0 = split * g.ksplit * (KT / KS);
-  const int ktiles = min(kt_all, kt0 + g.ksplit * (KT / KS)) - kt0;   // stages of this CTA's range
-  const int nacc = (ktiles + 1) / 2;                                   // accumulation rounds
+  const uint32_t items = (uint32_t)g.items;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       tc::mbar_init(&full_bar[s], 1);
       tc::mbar_init(&empty_bar[s], 1);
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < NBUF; ++b) {
       tc::mbar_init(&tfull_bar[b], 1);
-      tc::mbar_init(&tempty_bar[b], 4);   // one arrival per epilogue warp
+      tc::mbar_init(&tempty_bar[b], C_::EPI_WARPS);   // one arrival per epilogue warp
     }
     tc::mbar_init(&drain_bar, 1);
     tc::fence_mbar_init();
   }
   if (warp == 1) {
-    tc::tmem_alloc(&tmem_base, 2 * ACC_COLS);
+    tc::tmem_alloc(&tmem_base, TMEM_COLS);
     tc::tmem_relinquish();
-  }
-  if (threadIdx.x >= 64 && threadIdx.x < 64 + NT) {
-    const int j = threadIdx.x - 64;
-    const int64_t n = n0 + j;
-    noff[j] = (n < g.N) ? decode_off(g.no, n) : -1;
   }
   tc::fence_before();
   __syncthreads();
@@ -155,86 +296,96 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (lane == 0) {
       tc::prefetch_tmap(&tmA);
       tc::prefetch_tmap(&tmB);
-      int issued = 0;
+      uint32_t issued = 0;           // stages loaded so far
       bool aborted = false;
-      for (int kt = 0; kt < ktiles; ++kt) {
-        const int s = kt % STAGES;
-        const int use = kt / STAGES;
-        if (use > 0 && !tc::mbar_wait_abortable(&empty_bar[s], (use - 1) & 1, WAIT_CYCLES, vstatus)) {
-          atomicExch(g.status, PTN_ERR_TIMEOUT);
+      for (uint32_t w = blockIdx.x; w < items && !aborted; w += gridDim.x) {
+        const Item it = item_at<NT>(g, w);
+        if (*vstatus != 0) {         // an error elsewhere: the other warps see it in their waits
           aborted = true;
           break;
         }
-        uint8_t* st = smem + s * STAGE_BYTES;
-        tc::mbar_arrive_expect_tx(&full_bar[s], STAGE_BYTES);
-        const int kx = (kt0 + kt) * KS;
-        for (int p = 0; p < 2 * L; ++p)
-          tc::tma_load_3d(st + p * A_PLANE_BYTES, &tmA, &full_bar[s], kx, (int)m0, p);
-        for (int b = 0; b < 3 * L; ++b)
-          tc::tma_load_3d(st + A_STAGE_BYTES + b * B_BLOCK_BYTES, &tmB, &full_bar[s], kx, (int)n0, b);
-        ++issued;
+        for (int kt = 0; kt < it.stages; ++kt) {
+          const uint32_t s = issued % STAGES, use = issued / STAGES;
+          if (use > 0 && !tc::mbar_wait_abortable(&empty_bar[s], (use - 1) & 1, WAIT_CYCLES, vstatus)) {
+            atomicExch(g.status, PTN_ERR_TIMEOUT);
+            aborted = true;
+            break;
+          }
+          uint8_t* st = smem + s * STAGE_BYTES;
+          tc::mbar_arrive_expect_tx(&full_bar[s], STAGE_BYTES);
+          const int kx = (it.k0 + kt) * KS;
+          for (int p = 0; p < 2 * L; ++p)
+            tc::tma_load_3d(st + p * A_PLANE_BYTES, &tmA, &full_bar[s], kx, (int)it.m0, p);
+          for (int b = 0; b < 3 * L; ++b)
+            tc::tma_load_3d(st + A_STAGE_BYTES + b * B_BLOCK_BYTES, &tmB, &full_bar[s], kx, (int)it.n0, b);
+          ++issued;
+        }
       }
       if (aborted) {
         // Drain before the CTA gives up its shared memory: wait (bounded) for
         // the last load issued into each stage. A stage's phase for its last
         // use is the only one still to complete, so a completed one returns
         // at once.
-        for (int s = 0; s < STAGES && s < issued; ++s) {
-          const int kt_last = s + ((issued - 1 - s) / STAGES) * STAGES;
-          tc::mbar_wait(&full_bar[s], (uint32_t)((kt_last / STAGES) & 1), WAIT_CYCLES);
-        }
+        for (uint32_t s = 0; s < STAGES && s < issued; ++s)
+          tc::mbar_wait(&full_bar[s], ((issued - 1 - s) / STAGES) & 1, WAIT_CYCLES);
       }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    // Each K tile accumulates into a fresh TMEM buffer (two, alternating); the
-    // epilogue warps add the tile's partial sum into FP32 registers. The
+    // Each accumulation round goes into a fresh TMEM buffer (in turn); the
+    // epilogue warps add the round's partial sum into FP32 registers. The
     // tensor-core accumulator loses precision in proportion to the number of
-    // accumulations it absorbs, so this bounds that loss to one tile.
+    // accumulations it absorbs, so this bounds that loss to one round.
     if (lane == 0) {
       const uint32_t idesc = tc::idesc_bf16(MT, 2 * NT);
       bool aborted = false, any_mma = false;
-      for (int kt = 0; kt < ktiles; ++kt) {
-        const int s = kt % STAGES;
-        const int a = kt >> 1;                  // accumulation round: stages 2a, 2a + 1
-        const int b = a & 1, ub = a >> 1;
-        const bool round_start = (kt & 1) == 0;
-        if (round_start && ub > 0 &&
-            !tc::mbar_wait_abortable(&tempty_bar[b], (ub - 1) & 1, WAIT_CYCLES, vstatus)) {
-          atomicExch(g.status, PTN_ERR_TIMEOUT);
-          aborted = true;
-          break;
-        }
-        if (!tc::mbar_wait_abortable(&full_bar[s], (kt / STAGES) & 1, WAIT_CYCLES, vstatus)) {
-          atomicExch(g.status, PTN_ERR_TIMEOUT);
-          aborted = true;
-          break;
-        }
-        any_mma = true;
-        tc::fence_after();
-        const uint32_t sa = tc::smem_u32(smem + s * STAGE_BYTES);
-        const uint32_t sb = sa + A_STAGE_BYTES;
-        const uint32_t acc = tmem + (uint32_t)b * ACC_COLS;
-        bool first = round_start;
-        // smallest split products first, the leading (0, 0) product last
+      uint32_t stage = 0, round = 0;
+      for (uint32_t w = blockIdx.x; w < items && !aborted; w += gridDim.x) {
+        const int stages = item_at<NT>(g, w).stages;
+        for (int kt = 0; kt < stages; ++kt, ++stage) {
+          const uint32_t s = stage % STAGES;
+          const uint32_t b = round % NBUF, ub = round / NBUF;
+          const bool round_start = (kt & 1) == 0;
+          if (round_start && ub > 0 &&
+              !tc::mbar_wait_abortable(&tempty_bar[b], (ub - 1) & 1, WAIT_CYCLES, vstatus)) {
+            atomicExch(g.status, PTN_ERR_TIMEOUT);
+            aborted = true;
+            break;
+          }
+          if (!tc::mbar_wait_abortable(&full_bar[s], (stage / STAGES) & 1, WAIT_CYCLES, vstatus)) {
+            atomicExch(g.status, PTN_ERR_TIMEOUT);
+            aborted = true;
+            break;
+          }
+          any_mma = true;
+          tc::fence_after();
+          const uint32_t sa = tc::smem_u32(smem + s * STAGE_BYTES);
+          const uint32_t sb = sa + A_STAGE_BYTES;
+          const uint32_t acc = tmem + b * ACC_COLS;
+          bool first = round_start;
+          // smallest split products first, the leading (0, 0) product last
 #pragma unroll
-        for (int lvl = L - 1; lvl >= 0; --lvl) {
+          for (int lvl = L - 1; lvl >= 0; --lvl) {
 #pragma unroll
-          for (int i = 0; i <= lvl; ++i) {
-            const int j = lvl - i;
-            // A planes: 2i = Re level i, 2i+1 = Im level i.
-            // B level j at sb + 3j*B_BLOCK: window [Br; Bi] at +1 block, [-Bi; Br] at +0.
-            const uint64_t ar = tc::sdesc_sw32(sa + (2 * i) * A_PLANE_BYTES);
-            const uint64_t ai = tc::sdesc_sw32(sa + (2 * i + 1) * A_PLANE_BYTES);
-            const uint64_t bt = tc::sdesc_sw32(sb + (3 * j + 1) * B_BLOCK_BYTES);
-            const uint64_t bb = tc::sdesc_sw32(sb + (3 * j) * B_BLOCK_BYTES);
-            tc::mma_bf16(acc, ar, bt, idesc, first ? 0u : 1u);
-            tc::mma_bf16(acc, ai, bb, idesc, 1u);
-            first = false;
+            for (int i = 0; i <= lvl; ++i) {
+              const int j = lvl - i;
+              // A planes: 2i = Re level i, 2i+1 = Im level i.
+              // B level j at sb + 3j*B_BLOCK: window [Br; Bi] at +1 block, [-Bi; Br] at +0.
+              const uint64_t ar = tc::sdesc_sw32(sa + (2 * i) * A_PLANE_BYTES);
+              const uint64_t ai = tc::sdesc_sw32(sa + (2 * i + 1) * A_PLANE_BYTES);
+              const uint64_t bt = tc::sdesc_sw32(sb + (3 * j + 1) * B_BLOCK_BYTES);
+              const uint64_t bb = tc::sdesc_sw32(sb + (3 * j) * B_BLOCK_BYTES);
+              tc::mma_bf16(acc, ar, bt, idesc, first ? 0u : 1u);
+              tc::mma_bf16(acc, ai, bb, idesc, 1u);
+              first = false;
+            }
+          }
+          tc::mma_commit(&empty_bar[s]);
+          if (!round_start || kt == stages - 1) {
+            tc::mma_commit(&tfull_bar[b]);
+            ++round;
           }
         }
-        tc::mma_commit(&empty_bar[s]);
-        if (!round_start || kt == ktiles - 1) tc::mma_commit(&tfull_bar[b]);
       }
       if (aborted && any_mma) {
         // every MMA this thread issued completes before TMEM is freed
@@ -243,83 +394,121 @@ __global__ void __launch_bounds__(THREADS, 1)
       }
     }
   } else {
-    // ---------------- epilogue (warps 2..5) ----------------
+    // ---------------- epilogue (warps 2 ...) ----------------
     const int q = warp & 3;                 // TMEM lane quarter of this warp
+    const int c0 = ((warp - 2) >> 2) * EC;  // its columns
     const int row = q * 32 + lane;
-    const int64_t m = m0 + row;
     const uint32_t lane_off = (uint32_t)(q * 32) << 16;
-    float acc_re[NT], acc_im[NT];
-#pragma unroll
-    for (int i = 0; i < NT; ++i) {
-      acc_re[i] = 0.f;
-      acc_im[i] = 0.f;
-    }
+    uint32_t round = 0;
     bool ok = true;
-    for (int a = 0; a < nacc && ok; ++a) {
-      const int b = a & 1;
-      ok = tc::mbar_wait_abortable(&tfull_bar[b], (a >> 1) & 1, WAIT_CYCLES, vstatus);
-      if (!ok) break;
-      tc::fence_after();
-      const uint32_t tb = tmem + lane_off + (uint32_t)b * ACC_COLS;
-      // two loads in flight per wait (re and im of 16 columns)
+    for (uint32_t w = blockIdx.x; w < items && ok; w += gridDim.x) {
+      const Item it = item_at<NT>(g, w);
+      const int nacc = (it.stages + 1) / 2;                // accumulation rounds
+      const int64_t m = it.m0 + row, n0 = it.n0 + c0;
+      int64_t* noff = noff_s[warp - 2];
+      __syncwarp();                         // the tile before has been written
 #pragma unroll
-      for (int j0 = 0; j0 < NT; j0 += 16) {
-        uint32_t vr[16], vi[16];
-        tc::tmem_ld16_nowait(tb + (uint32_t)j0, vr);
-        tc::tmem_ld16_nowait(tb + (uint32_t)(NT + j0), vi);
-        tc::tmem_wait_ld();
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          acc_re[j0 + i] += __uint_as_float(vr[i]);
-          acc_im[j0 + i] += __uint_as_float(vi[i]);
-        }
-      }
-      tc::fence_before();
+      for (int j = lane; j < EC; j += 32) noff[j] = n0 + j < g.N ? decode_off32(g.no, (uint32_t)(n0 + j)) : -1;
       __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&tempty_bar[b]);
-    }
-    if (!ok) {
-      if (lane == 0) atomicExch(g.status, PTN_ERR_TIMEOUT);
-    } else if (m < g.M && g.splits > 1) {
-      // this K range's FP32 partial sums; splitk_reduce_kernel adds the ranges
-      float2* P = g.partial + ((int64_t)split * g.M + m) * g.N + n0;
+      const int64_t moff = m < g.M ? decode_off32(g.mo, (uint32_t)m) : 0;
+      float acc_re[EC], acc_im[EC];
 #pragma unroll
-      for (int i = 0; i < NT; ++i)
-        if (n0 + i < g.N) P[i] = make_float2(acc_re[i], acc_im[i]);
-    } else if (m < g.M) {
-      const int64_t moff = decode_off(g.mo, m);
-      if (g.out_kind == 0) {
-        double2* C = static_cast<double2*>(g.C);
+      for (int i = 0; i < EC; ++i) {
+        acc_re[i] = 0.f;
+        acc_im[i] = 0.f;
+      }
+      for (int a = 0; a < nacc; ++a, ++round) {
+        const uint32_t b = round % NBUF;
+        ok = __all_sync(0xffffffffu,
+                        tc::mbar_wait_abortable(&tfull_bar[b], (round / NBUF) & 1, WAIT_CYCLES, vstatus));
+        if (!ok) break;
+        tc::fence_after();
+        const uint32_t tb = tmem + lane_off + b * ACC_COLS + (uint32_t)c0;
+        // two loads in flight per wait (re and im of LC columns: 16, or 8 where eight
+        // epilogue warps leave 168 registers a thread)
+        constexpr int LC = NT > EC ? 8 : 16;
 #pragma unroll
-        for (int i = 0; i < NT; ++i) {
-          const int64_t no = noff[i];
-          if (no >= 0) C[moff + no] = make_double2((double)acc_re[i], (double)acc_im[i]);
+        for (int j0 = 0; j0 < EC; j0 += LC) {
+          uint32_t vr[LC], vi[LC];
+          tc::tmem_ld_nowait<LC>(tb + (uint32_t)j0, vr);
+          tc::tmem_ld_nowait<LC>(tb + (uint32_t)(NT + j0), vi);
+          tc::tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < LC; ++i) {
+            acc_re[j0 + i] += __uint_as_float(vr[i]);
+            acc_im[j0 + i] += __uint_as_float(vi[i]);
+          }
+        }
+        tc::fence_before();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&tempty_bar[b]);
+      }
+      if (!ok) {
+        if (lane == 0) atomicExch(g.status, PTN_ERR_TIMEOUT);
+        break;
+      }
+      const bool row_ok = m < g.M;
+      if (g.splits > 1) {
+        // this K range's FP32 partial sums; splitk_reduce_kernel adds the ranges
+        float2* P = g.partial + ((int64_t)it.split * g.M + m) * g.N + n0;
+        if (!row_ok) {
+        } else if (g.store == ST_ROW4) {
+#pragma unroll
+          for (int i = 0; i < EC; i += 4)
+            if (n0 + i < g.N)
+              st_global_32(P + i, __float_as_uint(acc_re[i]), __float_as_uint(acc_im[i]),
+                           __float_as_uint(acc_re[i + 1]), __float_as_uint(acc_im[i + 1]),
+                           __float_as_uint(acc_re[i + 2]), __float_as_uint(acc_im[i + 2]),
+                           __float_as_uint(acc_re[i + 3]), __float_as_uint(acc_im[i + 3]));
+        } else {
+#pragma unroll
+          for (int i = 0; i < EC; ++i)
+            if (n0 + i < g.N) P[i] = make_float2(acc_re[i], acc_im[i]);
+        }
+      } else if (g.out_kind == 0) {
+        double2* C = static_cast<double2*>(g.C) + moff;
+        if (!row_ok) {
+        } else if (g.store == ST_ROW2) {
+#pragma unroll
+          for (int i = 0; i < EC; i += 2) {
+            const int64_t no = noff[i];
+            if (i % 8 == 0 && no < 0) break;
+            if (no >= 0)
+              asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};" ::"l"(C + no), "d"((double)acc_re[i]),
+                           "d"((double)acc_im[i]), "d"((double)acc_re[i + 1]), "d"((double)acc_im[i + 1])
+                           : "memory");
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < EC; ++i) {
+            const int64_t no = noff[i];
+            if (i % 8 == 0 && no < 0) break;
+            if (no >= 0) C[no] = make_double2((double)acc_re[i], (double)acc_im[i]);
+          }
         }
       } else {
-        __nv_bfloat16* C = static_cast<__nv_bfloat16*>(g.C);
-        const int64_t ps = g.c_plane;
-#pragma unroll
-        for (int i = 0; i < NT; ++i) {
-          const int64_t no = noff[i];
-          if (no < 0) continue;
-          const int64_t o = moff + no;
-          float r = acc_re[i], v = acc_im[i];
-#pragma unroll
-          for (int lv = 0; lv < L; ++lv) {
-            const __nv_bfloat16 rb = __float2bfloat16_rn(r);
-            const __nv_bfloat16 ib = __float2bfloat16_rn(v);
-            C[(2 * lv) * ps + o] = rb;
-            C[(2 * lv + 1) * ps + o] = ib;
-            r -= __bfloat162float(rb);
-            v -= __bfloat162float(ib);
-          }
+        __nv_bfloat16* C = static_cast<__nv_bfloat16*>(g.C) + moff;
+        switch (g.store) {
+#define PTN_STORE(kind)                                                            \
+  case kind:                                                                       \
+    store_planes<L, kind>(C, g.c_plane, acc_re, acc_im, noff, row_ok);             \
+    break;
+          PTN_STORE(ST_ROW8)
+          PTN_STORE(ST_ROW4)
+          PTN_STORE(ST_ROW2)
+          PTN_STORE(ST_PAIR4)
+          PTN_STORE(ST_PAIR2)
+          PTN_STORE(ST_PAIR)
+#undef PTN_STORE
+          default:
+            store_planes<L, ST_ONE>(C, g.c_plane, acc_re, acc_im, noff, row_ok);
         }
       }
     }
   }
   tc::fence_before();
   __syncthreads();
-  if (warp == 1) tc::tmem_dealloc(tmem, 2 * ACC_COLS);
+  if (warp == 1) tc::tmem_dealloc(tmem, TMEM_COLS);
 }
 
 // ---- tensor maps ---------------------------------------------------------------------
@@ -621,6 +810,40 @@ static bool smallk_pairs_ok(const GemmArgs& g, int64_t M) {
   return true;
 }
 
+// How the tensor-core kernel's epilogue may write this output.
+static int store_kind(const GemmArgs& g) {
+  const OutModes &m = g.mo, &n = g.no;
+  auto all = [](const OutModes& o, int count, int64_t mult) {
+    for (int i = 0; i < count; ++i)
+      if (o.stride[i] % mult) return false;
+    return true;
+  };
+  const uintptr_t base = reinterpret_cast<uintptr_t>(g.C);
+  if (g.splits > 1) return g.N % 4 == 0 && reinterpret_cast<uintptr_t>(g.partial) % 32 == 0 ? ST_ROW4 : ST_ONE;
+  if (n.n < 1 || m.n < 1) return ST_ONE;
+  const int64_t ns = n.stride[n.n - 1], nd = n.dim[n.n - 1];
+  if (g.out_kind == 0)
+    return ns == 1 && nd % 2 == 0 && all(n, n.n - 1, 2) && all(m, m.n, 2) && base % 32 == 0 ? ST_ROW2 : ST_ONE;
+  // stores of v entries: aligned, and no group of columns goes past a run
+  auto fits = [&](int64_t v, int mcount, int64_t cols) {
+    return g.c_plane % v == 0 && base % (2 * v) == 0 && all(n, n.n - 1, v) && all(m, mcount, v) &&
+           (nd % cols == 0 || n.n == 1);
+  };
+  if (ns == 1) {
+    if (fits(8, m.n, 8)) return ST_ROW8;
+    if (fits(4, m.n, 4)) return ST_ROW4;
+    if (fits(2, m.n, 2)) return ST_ROW2;
+  }
+  // rows in runs of 32 and more are written a whole sector at a time as they are
+  // (131072 x 1280 x 256: 1.37 ms one by one, 1.59 in pairs)
+  if (m.stride[m.n - 1] != 1 || m.dim[m.n - 1] % 2 || m.dim[m.n - 1] >= 32) return ST_ONE;
+  if (ns == 2) {
+    if (fits(8, m.n - 1, 8)) return ST_PAIR4;
+    if (fits(4, m.n - 1, 4)) return ST_PAIR2;
+  }
+  return g.c_plane % 2 == 0 && base % 4 == 0 && all(m, m.n - 1, 2) && all(n, n.n, 2) ? ST_PAIR : ST_ONE;
+}
+
 // Sum of the split-K partial sums (compensated FP32, ranges in order: deterministic),
 // written like the GEMM epilogue: complex128 through the output modes, or as
 // BF16 level planes.
@@ -664,7 +887,7 @@ __global__ void splitk_reduce_kernel(const float2* __restrict__ partial, int spl
 
 // Split of the K range for an M x N x K product: (splits, K tiles per split).
 void split_plan(int64_t M, int64_t N, int64_t K, int64_t& splits, int64_t& ksplit) {
-  const int64_t tiles = ((M + MT - 1) / MT) * ((N + NT - 1) / NT);
+  const int64_t tiles = ((M + MT - 1) / MT) * ((N + 63) / 64);
   const int64_t kt_all = (K + KT - 1) / KT;
   splits = 1;
   ksplit = kt_all;
@@ -683,11 +906,19 @@ void split_plan(int64_t M, int64_t N, int64_t K, int64_t& splits, int64_t& kspli
 
 int fill_out(const ptn_modes& src, OutModes& dst) {
   if (src.n < 0 || src.n > PTN_MAX_MODES) return PTN_ERR_ARG;
-  dst.n = src.n;
+  dst.n = 0;
   for (int i = 0; i < src.n; ++i) {
     if (src.dim[i] <= 0) return PTN_ERR_ARG;
-    dst.dim[i] = src.dim[i];
-    dst.stride[i] = src.stride_c[i];
+    const int64_t dim = src.dim[i], stride = src.stride_c[i];
+    if (dim == 1) continue;
+    // a mode that continues the one before it is part of it
+    if (dst.n > 0 && dst.stride[dst.n - 1] == dim * stride) {
+      dst.dim[dst.n - 1] *= dim;
+      dst.stride[dst.n - 1] = stride;
+      continue;
+    }
+    dst.dim[dst.n] = dim;
+    dst.stride[dst.n++] = stride;
   }
   return PTN_OK;
 }
@@ -714,7 +945,9 @@ unsigned grid_for(int64_t n) {
 
 }  // namespace
 
-extern "C" int ptn_cgemm_smem_bytes(int32_t levels) { return levels == 3 ? Cfg<3>::SMEM : Cfg<2>::SMEM; }
+extern "C" int ptn_cgemm_smem_bytes(int32_t levels) {
+  return levels == 3 ? max(Cfg<3, 64>::SMEM, Cfg<3, 128>::SMEM) : max(Cfg<2, 64>::SMEM, Cfg<2, 128>::SMEM);
+}
 
 extern "C" int64_t ptn_cgemm_partial_bytes(int64_t M, int64_t N, int64_t K) {
   if (M < 1 || N < 1 || K < 1) return 0;
@@ -723,14 +956,37 @@ extern "C" int64_t ptn_cgemm_partial_bytes(int64_t M, int64_t N, int64_t K) {
   return splits > 1 ? splits * M * N * (int64_t)sizeof(float2) : 0;
 }
 
-template <int L>
-int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, unsigned grid, cudaStream_t st) {
+static int sm_count() {
+  static const int n = []() {
+    int dev = 0, v = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      return 0;
+    return v;
+  }();
+  return n;
+}
+
+template <int L, int NT>
+static int launch_gemm(const ptn_cgemm_desc* d, GemmArgs& g, int64_t tm, cudaStream_t st) {
   // once per process, thread-safe; a failure is returned on every call
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(cgemm_bf16_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<L>::SMEM);
-  if (attr != cudaSuccess) return PTN_ERR_LAUNCH;
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      cgemm_bf16_kernel<L, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<L, NT>::SMEM);
+  const int n_sm = sm_count();
+  if (attr != cudaSuccess || n_sm <= 0) return PTN_ERR_LAUNCH;
+  CUtensorMap ta, tb;
+  if (make_map_3d(&ta, d->A, (uint64_t)d->K, (uint64_t)d->M, 2 * L, (uint64_t)d->lda * 2,
+                  (uint64_t)d->a_plane * 2, KS, MT))
+    return PTN_ERR_ARG;
+  if (make_map_3d(&tb, d->Bx, (uint64_t)d->K, (uint64_t)d->N, 3 * L, (uint64_t)d->ldb * 2,
+                  (uint64_t)d->N * (uint64_t)d->ldb * 2, KS, NT))
+    return PTN_ERR_ARG;
+  const int64_t items = tm * ((d->N + NT - 1) / NT) * g.splits;
+  if (items > 0x7fffffffLL - n_sm) return PTN_ERR_UNSUPPORTED;
+  g.tiles_m = (int32_t)tm;
+  g.items = (int32_t)items;
   PTN_COUNT(1);
-  cgemm_bf16_kernel<L><<<grid, THREADS, Cfg<L>::SMEM, st>>>(ta, tb, g);
+  cgemm_bf16_kernel<L, NT><<<(unsigned)(items < n_sm ? items : n_sm), Cfg<L, NT>::THREADS, Cfg<L, NT>::SMEM, st>>>(
+      ta, tb, g);
   if (g.splits > 1) {
     PTN_COUNT(1);
     splitk_reduce_kernel<<<grid_for(g.M * g.N), 256, 0, st>>>(g.partial, g.splits, g.M, g.N, g.mo, g.no,
@@ -805,17 +1061,6 @@ extern "C" int ptn_cgemm_bf16x3(const ptn_cgemm_desc* d, void* stream) {
     }
     return ptn_launch_status();
   }
-  CUtensorMap ta, tb;
-  const int L = d->levels;
-  if (make_map_3d(&ta, d->A, (uint64_t)d->K, (uint64_t)d->M, 2 * L, (uint64_t)d->lda * 2,
-                  (uint64_t)d->a_plane * 2, KS, MT))
-    return PTN_ERR_ARG;
-  if (make_map_3d(&tb, d->Bx, (uint64_t)d->K, (uint64_t)d->N, 3 * L, (uint64_t)d->ldb * 2,
-                  (uint64_t)d->N * (uint64_t)d->ldb * 2, KS, NT))
-    return PTN_ERR_ARG;
-  const int64_t tm = (d->M + MT - 1) / MT, tn = (d->N + NT - 1) / NT;
-  g.tiles_n = tn;
-  g.tiles = tm * tn;
   int64_t splits = 1, ksplit = (d->K + KT - 1) / KT;
   if (d->partial) {
     int64_t s_, k_;
@@ -829,9 +1074,19 @@ extern "C" int ptn_cgemm_bf16x3(const ptn_cgemm_desc* d, void* stream) {
   g.splits = (int32_t)splits;
   g.ksplit = (int32_t)ksplit;
   g.partial = static_cast<float2*>(d->partial);
-  if (tm * tn * splits > 0x7fffffffLL) return PTN_ERR_UNSUPPORTED;
-  const unsigned grid = (unsigned)(tm * tn * splits);
-  return L == 3 ? launch_gemm<3>(ta, tb, g, grid, ptn_stream(stream)) : launch_gemm<2>(ta, tb, g, grid, ptn_stream(stream));
+  g.store = store_kind(g);
+  // 128 columns or 64: the waves of the launch times a tile's cost. A tile of 128
+  // columns takes about 1.5 times one of 64: 163840 x 256 x 1280 at 1500 TFLOP/s in wide
+  // tiles, 131072 x 64 x 256 at 790 in narrow ones, of whose time a third is the start
+  // and the end.
+  const int64_t tm = (d->M + MT - 1) / MT;
+  const int64_t n_sm = sm_count() > 0 ? sm_count() : 1;
+  const int64_t w64 = (tm * ((d->N + 63) / 64) * splits + n_sm - 1) / n_sm;
+  const int64_t w128 = (tm * ((d->N + 127) / 128) * splits + n_sm - 1) / n_sm;
+  const bool wide = 3 * w128 < 2 * w64;
+  cudaStream_t st = ptn_stream(stream);
+  if (d->levels == 3) return wide ? launch_gemm<3, 128>(d, g, tm, st) : launch_gemm<3, 64>(d, g, tm, st);
+  return wide ? launch_gemm<2, 128>(d, g, tm, st) : launch_gemm<2, 64>(d, g, tm, st);
 }
 
 extern "C" int ptn_to_planes(const ptn_convert_desc* d, void* stream) {
