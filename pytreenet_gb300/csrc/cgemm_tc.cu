@@ -28,6 +28,8 @@
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 #include "ptn_common.cuh"
 #include "tc_ptx.cuh"
 
@@ -114,12 +116,12 @@ __device__ __forceinline__ int64_t decode_off(const OutModes& md, int64_t idx) {
 // The same for an index and extents below 2^31.
 __device__ __forceinline__ int64_t decode_off32(const OutModes& md, uint32_t idx) {
   int64_t o = 0;
-  for (int d = md.n - 1; d >= 0; --d) {
+  for (int d = md.n - 1; d > 0; --d) {
     const uint32_t dim = (uint32_t)md.dim[d], q = idx / dim;
     o += (int64_t)(idx - q * dim) * md.stride[d];
     idx = q;
   }
-  return o;
+  return md.n > 0 ? o + (int64_t)idx * md.stride[0] : 0;   // idx is in range: no division for the first
 }
 
 // Work items (K range, tile): CTA b takes b, b + gridDim.x, ... Tiles of a row block of
@@ -544,13 +546,10 @@ int make_map_3d(CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, ui
 }
 
 // ---- conversions ---------------------------------------------------------------------
-// planes[p][m * lda + k] <- split(src[off_m(m) + off_k(k)]) for the complex128 source.
 // x ~ out[0] + ... + out[L-1] in BF16 pieces. Only the first remainder needs
 // double precision: x - bf16(x) is exact in FP64 (Sterbenz) and is rounded
 // once to FP32 (error <= 2^-32 |x|, below the 2^-25 |x| the three pieces
-// leave); the later pieces are split in FP32. GB300 issues FP64 at 1/64 of the
-// FP32 rate, and a split done wholly in FP64 made the conversion of the χ=256
-// root vector FP64-bound (0.93 ms for 33.5 M entries).
+// leave); the later pieces are split in FP32.
 __device__ __forceinline__ void split_levels(double x, int L, __nv_bfloat16* out) {
   const __nv_bfloat16 b0 = __double2bfloat16(x);
   out[0] = b0;
@@ -561,87 +560,161 @@ __device__ __forceinline__ void split_levels(double x, int L, __nv_bfloat16* out
     r -= __bfloat162float(b);
   }
 }
+// Values outside [2^-60, 2^120): the pieces may leave FP32's normal range.
+template <int L>
+__device__ __noinline__ void split_far(double x, uint32_t* out) {
+  __nv_bfloat16 b[3];
+  split_levels(x, L, b);
+#pragma unroll
+  for (int lv = 0; lv < L; ++lv) out[lv] = (uint32_t)__bfloat16_as_ushort(b[lv]);
+}
+// The same pieces with one instruction at FP64 rate, the conversion of the remainder,
+// instead of five: a warp instruction of the FP64 pipe takes an SM 16 cycles, and the
+// conversion of a 4.2 M entry vector with them 91 us where its traffic takes 17. The
+// leading piece is the 53-bit mantissa rounded at its eighth bit in integers; the bits
+// below, less one unit if it was rounded up, are the exact remainder.
+// flip: 0, or the sign bit to convert -x.
+template <int L>
+__device__ __forceinline__ void split_bits(double x, uint32_t flip, uint32_t (&out)[L]) {
+  const uint32_t h = (uint32_t)__double2hiint(x) ^ flip, lo = (uint32_t)__double2loint(x), ah = h & 0x7fffffffu;
+  const int e = (int)(ah >> 20);
+  if ((unsigned)(e - 963) >= 180u && (ah | lo) != 0u) {
+    split_far<L>(__hiloint2double((int)h, (int)lo), out);
+    return;
+  }
+  const bool zero = (ah | lo) == 0u;
+  const uint32_t tail = ah & 0x1fffu;
+  const uint32_t up = (tail > 0x1000u || (tail == 0x1000u && (lo != 0u || (ah & 0x2000u)))) ? 1u : 0u;
+  // exponent rebased to FP32's, above the seven mantissa bits that are kept
+  const uint32_t b0 = zero ? 0u : (ah >> 13) - (896u << 7) + up;
+  out[0] = b0 | (h >> 31 << 15);
+  const int rh = (int)tail - (int)(up << 13);
+  const long long rem = ((long long)rh << 32) | lo;
+  // times 2^(e - 1075) with x's sign; an exact zero stays +0
+  const float scale = __uint_as_float(((uint32_t)(e - 948) << 23) | (h & 0x80000000u));
+  float r = zero || rem == 0 ? 0.f : __ll2float_rn(rem) * scale;
+#pragma unroll
+  for (int lv = 1; lv < L; ++lv) out[lv] = take_bf16(r);
+}
 
-__global__ void to_planes_kernel(const double2* __restrict__ src, OutModes mm, OutModes km, int64_t M, int64_t K,
-                                 int64_t lda, int64_t plane, int conj, int L, __nv_bfloat16* __restrict__ dst) {
-  const int64_t total = M * K;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t m = e / K, k = e - (e / K) * K;
-    double2 v = src[decode_off(mm, m) + decode_off(km, k)];
-    if (conj) v.y = -v.y;
-    __nv_bfloat16 re[3], im[3];
-    split_levels(v.x, L, re);
-    split_levels(v.y, L, im);
-    const int64_t o = m * lda + k;
-    for (int lv = 0; lv < L; ++lv) {
-      dst[(2 * lv) * plane + o] = re[lv];
-      dst[(2 * lv + 1) * plane + o] = im[lv];
+// The pieces of two neighbouring entries, one word per level.
+template <int L>
+__device__ __forceinline__ void split_pair(double x, double y, uint32_t flip, uint32_t (&w)[L]) {
+  uint32_t a[L], b[L];
+  split_bits<L>(x, flip, a);
+  split_bits<L>(y, flip, b);
+#pragma unroll
+  for (int lv = 0; lv < L; ++lv) w[lv] = a[lv] | b[lv] << 16;
+}
+
+struct ConvArgs {
+  const double2* src;
+  OutModes rm, km;               // rows and K index of the operand
+  int64_t rows, K, ld, plane;
+  int conj;
+  int words;                     // rows and planes start on 4 bytes
+  int64_t kstep;                 // source step from an even K index to the next, 0: look it up
+  __nv_bfloat16* dst;
+};
+// V (2 or 4) entries of row r from K index k into the operand's layout: 2 L planes of A
+// (Re_0, Im_0, ...) or, EXPAND, B's blocks [level][-Bi, Br, Bi][row][k]. With V = 2 the
+// second may lie past the end, and rows may start on 2 bytes.
+template <int L, bool EXPAND, int V>
+__device__ __forceinline__ void put_split(const ConvArgs& c, int64_t r, int64_t k, const double2 (&v)[V]) {
+  uint32_t re[V / 2][L], im[V / 2][L];
+  const uint32_t flip = c.conj ? 0x80000000u : 0u;
+#pragma unroll
+  for (int i = 0; i < V / 2; ++i) {
+    split_pair<L>(v[2 * i].x, v[2 * i + 1].x, 0u, re[i]);
+    split_pair<L>(v[2 * i].y, v[2 * i + 1].y, flip, im[i]);
+  }
+  __nv_bfloat16* p = c.dst + r * c.ld + k;
+  const int64_t blk = EXPAND ? c.rows * c.ld : c.plane;
+  auto put = [&](int64_t plane, uint32_t a, uint32_t b) {
+    __nv_bfloat16* q = p + plane * blk;
+    if (V == 4) {
+      *reinterpret_cast<uint2*>(q) = make_uint2(a, b);
+    } else if (c.words && k + 1 < c.K) {
+      *reinterpret_cast<uint32_t*>(q) = a;
+    } else {
+      q[0] = __ushort_as_bfloat16((unsigned short)a);
+      if (k + 1 < c.K) q[1] = __ushort_as_bfloat16((unsigned short)(a >> 16));
+    }
+  };
+#pragma unroll
+  for (int lv = 0; lv < L; ++lv) {
+    const uint32_t r0 = re[0][lv], r1 = re[V / 2 - 1][lv], i0 = im[0][lv], i1 = im[V / 2 - 1][lv];
+    if (EXPAND) {
+      put(3 * lv, i0 ^ 0x80008000u, i1 ^ 0x80008000u);
+      put(3 * lv + 1, r0, r1);
+      put(3 * lv + 2, i0, i1);
+    } else {
+      put(2 * lv, r0, r1);
+      put(2 * lv + 1, i0, i1);
     }
   }
 }
 
-// The same conversion through a 32 x 32 shared-memory tile, for operands
+// planes[p][m * lda + k] <- split(src[off_m(m) + off_k(k)]); a thread takes two
+// neighbouring K indices, or four where rows and K runs allow 8-byte stores. WIDE:
+// 64-bit indices.
+template <bool WIDE>
+__device__ __forceinline__ int64_t mode_off(const OutModes& md, int64_t idx) {
+  return WIDE ? decode_off(md, idx) : decode_off32(md, (uint32_t)idx);
+}
+template <int L, bool EXPAND, bool WIDE, int V>
+__global__ void __launch_bounds__(256) convert_kernel(const ConvArgs c) {
+  using I = typename std::conditional<WIDE, int64_t, uint32_t>::type;
+  const I kp = (I)((c.K + V - 1) / V), total = (I)c.rows * kp;
+  for (I e = (I)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (I)gridDim.x * blockDim.x) {
+    const I r = e / kp, k = V * (e - r * kp);
+    const double2* src = c.src + mode_off<WIDE>(c.rm, r) + mode_off<WIDE>(c.km, k);
+    double2 v[V];
+    v[0] = src[0];
+    if (V == 4 || c.kstep != 0) {
+#pragma unroll
+      for (int i = 1; i < V; ++i) v[i] = src[i * c.kstep];
+    } else {
+      v[1] = make_double2(0.0, 0.0);
+      if ((int64_t)k + 1 < c.K) v[1] = c.src[mode_off<WIDE>(c.rm, r) + mode_off<WIDE>(c.km, (int64_t)k + 1)];
+    }
+    put_split<L, EXPAND, V>(c, r, k, v);
+  }
+}
+
+// The same conversion through a 32 x 64 shared-memory tile, for operands
 // whose rows are contiguous in the source while the K index is not (the first
 // step of a matvec contracting the parent leg reads x with a stride of the
 // whole rest of the tensor): the tile is read with the row index across the
 // threads and written with the K index across them, so both sides coalesce.
-// Each element is converted exactly as in to_planes_kernel.
-__global__ void __launch_bounds__(256) to_planes_tiled_kernel(const double2* __restrict__ src, OutModes mm,
-                                                              OutModes km, int64_t M, int64_t K, int64_t lda,
-                                                              int64_t plane, int conj, int L,
-                                                              __nv_bfloat16* __restrict__ dst) {
-  __shared__ double2 tile[32][33];
+// Measured, with split_bits: 32768 x 128 (the vector of a 3-leg site at bond 128) 90
+// -> 40 us, 131072 x 256 687 -> 232 (940 MB), and along K 584 -> 216.
+constexpr int TILE_K = 64;
+template <int L, bool EXPAND, bool WIDE>
+__global__ void __launch_bounds__(256) convert_tiled_kernel(const ConvArgs c) {
+  __shared__ double2 tile[TILE_K][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int64_t tiles_k = (K + 31) / 32;
-  const int64_t tiles = ((M + 31) / 32) * tiles_k;
+  const int64_t tiles_k = (c.K + TILE_K - 1) / TILE_K;
+  const int64_t tiles = ((c.rows + 31) / 32) * tiles_k;
   for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-    const int64_t m0 = (t / tiles_k) * 32, k0 = (t - (t / tiles_k) * tiles_k) * 32;
-    for (int r = ty; r < 32; r += 8) {
-      const int64_t m = m0 + tx, k = k0 + r;
-      double2 v = make_double2(0.0, 0.0);
-      if (m < M && k < K) v = src[decode_off(mm, m) + decode_off(km, k)];
-      tile[r][tx] = v;
+    const int64_t m0 = (t / tiles_k) * 32, k0 = (t - (t / tiles_k) * tiles_k) * TILE_K;
+    const bool row = m0 + tx < c.rows;
+    const double2* src = c.src + (row ? mode_off<WIDE>(c.rm, m0 + tx) : 0);
+#pragma unroll
+    for (int q = 0; q < TILE_K / 8; ++q) {
+      const int64_t k = k0 + ty + 8 * q;
+      tile[ty + 8 * q][tx] = row && k < c.K ? src[mode_off<WIDE>(c.km, k)] : make_double2(0.0, 0.0);
     }
     __syncthreads();
+#pragma unroll
     for (int r = ty; r < 32; r += 8) {
-      const int64_t m = m0 + r, k = k0 + tx;
-      if (m < M && k < K) {
-        double2 v = tile[tx][r];
-        if (conj) v.y = -v.y;
-        __nv_bfloat16 re[3], im[3];
-        split_levels(v.x, L, re);
-        split_levels(v.y, L, im);
-        const int64_t o = m * lda + k;
-        for (int lv = 0; lv < L; ++lv) {
-          dst[(2 * lv) * plane + o] = re[lv];
-          dst[(2 * lv + 1) * plane + o] = im[lv];
-        }
+      const int64_t m = m0 + r, k = k0 + 2 * tx;
+      if (m < c.rows && k < c.K) {
+        const double2 v[2] = {tile[2 * tx][r], tile[2 * tx + 1][r]};
+        put_split<L, EXPAND, 2>(c, m, k, v);
       }
     }
     __syncthreads();
-  }
-}
-
-// Bx[level][block][n][k]: block 0 = -Bi, 1 = Br, 2 = Bi.
-__global__ void expand_b_kernel(const double2* __restrict__ src, OutModes nm, OutModes km, int64_t N, int64_t K,
-                                int64_t ldb, int conj, int L, __nv_bfloat16* __restrict__ dst) {
-  const int64_t total = N * K;
-  const int64_t blk = N * ldb;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t n = e / K, k = e - (e / K) * K;
-    double2 v = src[decode_off(nm, n) + decode_off(km, k)];
-    if (conj) v.y = -v.y;
-    __nv_bfloat16 re[3], im[3];
-    split_levels(v.x, L, re);
-    split_levels(v.y, L, im);
-    const int64_t o = n * ldb + k;
-    for (int lv = 0; lv < L; ++lv) {
-      dst[(3 * lv + 0) * blk + o] = __hneg(im[lv]);
-      dst[(3 * lv + 1) * blk + o] = re[lv];
-      dst[(3 * lv + 2) * blk + o] = im[lv];
-    }
   }
 }
 
@@ -904,34 +977,36 @@ void split_plan(int64_t M, int64_t N, int64_t K, int64_t& splits, int64_t& kspli
   }
 }
 
+// A mode that continues the one before it is part of it.
+void add_mode(OutModes& m, int64_t dim, int64_t stride) {
+  if (dim == 1) return;
+  if (m.n > 0 && m.stride[m.n - 1] == dim * stride) {
+    m.dim[m.n - 1] *= dim;
+    m.stride[m.n - 1] = stride;
+    return;
+  }
+  m.dim[m.n] = dim;
+  m.stride[m.n++] = stride;
+}
+
 int fill_out(const ptn_modes& src, OutModes& dst) {
   if (src.n < 0 || src.n > PTN_MAX_MODES) return PTN_ERR_ARG;
   dst.n = 0;
   for (int i = 0; i < src.n; ++i) {
     if (src.dim[i] <= 0) return PTN_ERR_ARG;
-    const int64_t dim = src.dim[i], stride = src.stride_c[i];
-    if (dim == 1) continue;
-    // a mode that continues the one before it is part of it
-    if (dst.n > 0 && dst.stride[dst.n - 1] == dim * stride) {
-      dst.dim[dst.n - 1] *= dim;
-      dst.stride[dst.n - 1] = stride;
-      continue;
-    }
-    dst.dim[dst.n] = dim;
-    dst.stride[dst.n++] = stride;
+    add_mode(dst, src.dim[i], src.stride_c[i]);
   }
   return PTN_OK;
 }
 
 int fill_src(const ptn_modes& src, OutModes& dst, int64_t& total) {
   if (src.n < 0 || src.n > PTN_MAX_MODES) return PTN_ERR_ARG;
-  dst.n = src.n;
+  dst.n = 0;
   total = 1;
   for (int i = 0; i < src.n; ++i) {
     if (src.dim[i] <= 0) return PTN_ERR_ARG;
-    dst.dim[i] = src.dim[i];
-    dst.stride[i] = src.stride_a[i];
     total *= src.dim[i];
+    add_mode(dst, src.dim[i], src.stride_a[i]);
   }
   return PTN_OK;
 }
@@ -1089,38 +1164,59 @@ extern "C" int ptn_cgemm_bf16x3(const ptn_cgemm_desc* d, void* stream) {
   return wide ? launch_gemm<2, 128>(d, g, tm, st) : launch_gemm<2, 64>(d, g, tm, st);
 }
 
-extern "C" int ptn_to_planes(const ptn_convert_desc* d, void* stream) {
-  if (!d || !d->src || !d->dst || (d->levels != 2 && d->levels != 3)) return PTN_ERR_ARG;
-  OutModes mm, km;
-  int64_t M, K;
-  if (fill_src(d->rows, mm, M) || fill_src(d->cols, km, K)) return PTN_ERR_ARG;
-  if (d->ld < K) return PTN_ERR_ARG;
-  PTN_COUNT(1);
+template <int L, bool EXPAND>
+static int convert(ConvArgs& c, cudaStream_t st) {
+  // 32-bit indices unless they overflow (the grid's stride included)
+  const bool wide = c.rows > 0x3fffffffLL || c.K > 0x3fffffffLL || c.rows * ((c.K + 1) / 2) > 0x7fffffffLL;
+  const OutModes &rm = c.rm, &km = c.km;
   // innermost (fastest) source strides of the row and K indices
-  const int64_t sm = mm.n > 0 ? mm.stride[mm.n - 1] : 0, sk = km.n > 0 ? km.stride[km.n - 1] : 0;
-  const int64_t asm_ = sm < 0 ? -sm : sm, ask = sk < 0 ? -sk : sk;
-  if (M >= 32 && K >= 32 && asm_ <= 2 && ask > 2) {
-    const int64_t tiles = ((M + 31) / 32) * ((K + 31) / 32);
-    to_planes_tiled_kernel<<<(unsigned)(tiles < 152 * 16 ? tiles : 152 * 16), 256, 0, ptn_stream(stream)>>>(
-        static_cast<const double2*>(d->src), mm, km, M, K, d->ld, d->plane, d->conj, d->levels,
-        static_cast<__nv_bfloat16*>(d->dst));
+  const int64_t sr = rm.n > 0 ? rm.stride[rm.n - 1] : 0, sk = km.n > 0 ? km.stride[km.n - 1] : 0;
+  const int64_t asr = sr < 0 ? -sr : sr, ask = sk < 0 ? -sk : sk;
+  PTN_COUNT(1);
+  // fewer tiles leave the GPU idle, and so small a source is read from L2 anyway
+  // (40 x 40: 14 us tiled, 10 not; 512 x 256: 11 and 16)
+  const int64_t tiles = ((c.rows + 31) / 32) * ((c.K + TILE_K - 1) / TILE_K);
+  if (c.rows >= 32 && c.K >= 32 && asr <= 2 && ask > 2 && tiles >= 32) {
+    const unsigned grid = (unsigned)(tiles < 152 * 16 ? tiles : 152 * 16);
+    if (wide) convert_tiled_kernel<L, EXPAND, true><<<grid, 256, 0, st>>>(c);
+    else convert_tiled_kernel<L, EXPAND, false><<<grid, 256, 0, st>>>(c);
     return ptn_launch_status();
   }
-  to_planes_kernel<<<grid_for(M * K), 256, 0, ptn_stream(stream)>>>(
-      static_cast<const double2*>(d->src), mm, km, M, K, d->ld, d->plane, d->conj, d->levels,
-      static_cast<__nv_bfloat16*>(d->dst));
+  // groups of K indices lie in one run of the innermost mode
+  const int64_t run = km.n > 0 ? km.dim[km.n - 1] : 1;
+  const bool four = run % 4 == 0 && c.ld % 4 == 0 && c.plane % 4 == 0 && reinterpret_cast<uintptr_t>(c.dst) % 8 == 0;
+  const unsigned grid = grid_for(c.rows * ((c.K + (four ? 3 : 1)) / (four ? 4 : 2)));
+  c.kstep = run % 2 == 0 ? sk : 0;
+  if (wide) convert_kernel<L, EXPAND, true, 2><<<grid, 256, 0, st>>>(c);
+  else if (four) convert_kernel<L, EXPAND, false, 4><<<grid, 256, 0, st>>>(c);
+  else convert_kernel<L, EXPAND, false, 2><<<grid, 256, 0, st>>>(c);
   return ptn_launch_status();
 }
 
-extern "C" int ptn_expand_b(const ptn_convert_desc* d, void* stream) {
+static int convert_args(const ptn_convert_desc* d, ConvArgs& c) {
   if (!d || !d->src || !d->dst || (d->levels != 2 && d->levels != 3)) return PTN_ERR_ARG;
-  OutModes nm, km;
-  int64_t N, K;
-  if (fill_src(d->rows, nm, N) || fill_src(d->cols, km, K)) return PTN_ERR_ARG;
-  if (d->ld < K) return PTN_ERR_ARG;
-  PTN_COUNT(1);
-  expand_b_kernel<<<grid_for(N * K), 256, 0, ptn_stream(stream)>>>(
-      static_cast<const double2*>(d->src), nm, km, N, K, d->ld, d->conj, d->levels,
-      static_cast<__nv_bfloat16*>(d->dst));
-  return ptn_launch_status();
+  if (fill_src(d->rows, c.rm, c.rows) || fill_src(d->cols, c.km, c.K)) return PTN_ERR_ARG;
+  if (d->ld < c.K) return PTN_ERR_ARG;
+  c.src = static_cast<const double2*>(d->src);
+  c.dst = static_cast<__nv_bfloat16*>(d->dst);
+  c.ld = d->ld;
+  c.plane = d->plane;
+  c.conj = d->conj;
+  c.kstep = 0;
+  c.words = d->ld % 2 == 0 && d->plane % 2 == 0 && reinterpret_cast<uintptr_t>(d->dst) % 4 == 0;
+  return PTN_OK;
+}
+
+extern "C" int ptn_to_planes(const ptn_convert_desc* d, void* stream) {
+  ConvArgs c;
+  const int st = convert_args(d, c);
+  if (st != PTN_OK) return st;
+  return d->levels == 3 ? convert<3, false>(c, ptn_stream(stream)) : convert<2, false>(c, ptn_stream(stream));
+}
+
+extern "C" int ptn_expand_b(const ptn_convert_desc* d, void* stream) {
+  ConvArgs c;
+  const int st = convert_args(d, c);
+  if (st != PTN_OK) return st;
+  return d->levels == 3 ? convert<3, true>(c, ptn_stream(stream)) : convert<2, true>(c, ptn_stream(stream));
 }
