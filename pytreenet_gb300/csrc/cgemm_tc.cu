@@ -797,17 +797,32 @@ __global__ void __launch_bounds__(SMALLK_T)
   }
 }
 
+// d = a b + c in both halves of a register pair.
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  return (unsigned long long)__float_as_uint(y) << 32 | __float_as_uint(x);
+}
+
 // The same product for BF16-plane outputs whose rows come in adjacent pairs:
 // thread t computes rows 2t and 2t + 1 and stores each plane entry of the pair
 // as one 4-byte bf16x2 (the host checks that the innermost row mode has
 // output stride 1 and an even extent and that every other stride is even, so
 // the pair is adjacent and 4-byte aligned). Half the store instructions, and a
 // warp writes 128 contiguous bytes per plane. Same arithmetic per output.
-template <int KK>
+//
+// 16777216 x 50 x 10 reads 2 GB and writes 10 GB (1.8 ms at the copy rate) and was bound
+// by instruction issue: 2.72 ms. So both rows share an instruction (FP32 pairs), a pair's
+// entries of a plane, contiguous where rows are KK apart (DENSE), come in 8-byte
+// loads, and both rows of a piece are rounded together: 2.05 ms.
+template <int KK, int L, bool DENSE>
 __global__ void __launch_bounds__(SMALLK_T)
     cgemm_smallk_pair_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, int64_t a_plane,
-                             const __nv_bfloat16* __restrict__ Bx, int64_t ldb, GemmArgs g, int L) {
-  __shared__ float2 sB[SMALLK_MAX_N * KK];
+                             const __nv_bfloat16* __restrict__ Bx, int64_t ldb, GemmArgs g) {
+  __shared__ ulonglong2 sB[SMALLK_MAX_N * KK];       // (Re, Re), (Im, Im)
   __shared__ int64_t noff[SMALLK_MAX_N];
   if (*(volatile int32_t*)g.status != 0) return;
   const int N = (int)g.N;
@@ -819,54 +834,81 @@ __global__ void __launch_bounds__(SMALLK_T)
       re += __bfloat162float(Bx[(3 * lv + 1) * blk + (int64_t)n * ldb + kk]);
       im += __bfloat162float(Bx[(3 * lv + 2) * blk + (int64_t)n * ldb + kk]);
     }
-    sB[n * KK + kk] = make_float2(re, im);
+    sB[n * KK + kk] = make_ulonglong2(pack2(re, re), pack2(im, im));
   }
-  for (int n = threadIdx.x; n < N; n += SMALLK_T) noff[n] = decode_off(g.no, n);
+  for (int n = threadIdx.x; n < N; n += SMALLK_T) noff[n] = decode_off32(g.no, (uint32_t)n);
   __syncthreads();
   const int64_t pairs = g.M / 2;
   for (int64_t pr = blockIdx.x * (int64_t)SMALLK_T + threadIdx.x; pr < pairs;
        pr += (int64_t)gridDim.x * SMALLK_T) {
     const int64_t m = 2 * pr;
-    float2 a0[KK], a1[KK];
+    // row m in the low halves, row m + 1 in the high ones
+    unsigned long long ax[KK], ay[KK], nay[KK];
 #pragma unroll
-    for (int kk = 0; kk < KK; ++kk) {
-      float r0 = 0.f, i0 = 0.f, r1 = 0.f, i1 = 0.f;
+    for (int part = 0; part < 2; ++part) {
+      float v0[KK], v1[KK];
+#pragma unroll
+      for (int kk = 0; kk < KK; ++kk) v0[kk] = v1[kk] = 0.f;
+#pragma unroll
       for (int lv = 0; lv < L; ++lv) {
-        r0 += __bfloat162float(A[(2 * lv) * a_plane + m * lda + kk]);
-        i0 += __bfloat162float(A[(2 * lv + 1) * a_plane + m * lda + kk]);
-        r1 += __bfloat162float(A[(2 * lv) * a_plane + (m + 1) * lda + kk]);
-        i1 += __bfloat162float(A[(2 * lv + 1) * a_plane + (m + 1) * lda + kk]);
+        const __nv_bfloat16* p = A + (2 * lv + part) * a_plane + m * lda;
+        if (DENSE) {
+          uint32_t w[KK];                            // entries 2 i and 2 i + 1 of the 2 KK
+#pragma unroll
+          for (int i = 0; i < KK / 2; ++i) {
+            const uint2 u = __ldg(reinterpret_cast<const uint2*>(p) + i);
+            w[2 * i] = u.x;
+            w[2 * i + 1] = u.y;
+          }
+#pragma unroll
+          for (int kk = 0; kk < KK; ++kk) {
+            const uint32_t x = w[kk / 2], y = w[KK / 2 + kk / 2];
+            v0[kk] += __uint_as_float(kk & 1 ? x & 0xffff0000u : x << 16);
+            v1[kk] += __uint_as_float(kk & 1 ? y & 0xffff0000u : y << 16);
+          }
+        } else {
+#pragma unroll
+          for (int kk = 0; kk < KK; ++kk) {
+            v0[kk] += __bfloat162float(p[kk]);
+            v1[kk] += __bfloat162float(p[lda + kk]);
+          }
+        }
       }
-      a0[kk] = make_float2(r0, i0);
-      a1[kk] = make_float2(r1, i1);
-    }
-    const int64_t moff = decode_off(g.mo, m);
-    __nv_bfloat16* C = static_cast<__nv_bfloat16*>(g.C);
-    for (int n = 0; n < N; ++n) {
-      float cr0 = 0.f, ci0 = 0.f, cr1 = 0.f, ci1 = 0.f;
 #pragma unroll
       for (int kk = 0; kk < KK; ++kk) {
-        const float2 b = sB[n * KK + kk];
-        cr0 = fmaf(a0[kk].x, b.x, cr0);
-        cr0 = fmaf(-a0[kk].y, b.y, cr0);
-        ci0 = fmaf(a0[kk].x, b.y, ci0);
-        ci0 = fmaf(a0[kk].y, b.x, ci0);
-        cr1 = fmaf(a1[kk].x, b.x, cr1);
-        cr1 = fmaf(-a1[kk].y, b.y, cr1);
-        ci1 = fmaf(a1[kk].x, b.y, ci1);
-        ci1 = fmaf(a1[kk].y, b.x, ci1);
+        if (part == 0) {
+          ax[kk] = pack2(v0[kk], v1[kk]);
+        } else {
+          ay[kk] = pack2(v0[kk], v1[kk]);
+          nay[kk] = pack2(-v0[kk], -v1[kk]);
+        }
       }
-      const int64_t o = moff + noff[n];
-      for (int lv = 0; lv < L; ++lv) {
-        const __nv_bfloat16 rb0 = __float2bfloat16_rn(cr0), ib0 = __float2bfloat16_rn(ci0);
-        const __nv_bfloat16 rb1 = __float2bfloat16_rn(cr1), ib1 = __float2bfloat16_rn(ci1);
-        *reinterpret_cast<__nv_bfloat162*>(C + (2 * lv) * g.c_plane + o) = __halves2bfloat162(rb0, rb1);
-        *reinterpret_cast<__nv_bfloat162*>(C + (2 * lv + 1) * g.c_plane + o) = __halves2bfloat162(ib0, ib1);
-        cr0 -= __bfloat162float(rb0);
-        ci0 -= __bfloat162float(ib0);
-        cr1 -= __bfloat162float(rb1);
-        ci1 -= __bfloat162float(ib1);
+    }
+    __nv_bfloat16* C = static_cast<__nv_bfloat16*>(g.C) + decode_off32(g.mo, (uint32_t)m);
+    for (int n = 0; n < N; ++n) {
+      unsigned long long cr = 0ull, ci = 0ull;
+#pragma unroll
+      for (int kk = 0; kk < KK; ++kk) {
+        const ulonglong2 b = sB[n * KK + kk];
+        cr = fma2(ax[kk], b.x, cr);
+        cr = fma2(nay[kk], b.y, cr);
+        ci = fma2(ax[kk], b.y, ci);
+        ci = fma2(ay[kk], b.x, ci);
       }
+      __nv_bfloat16* p = C + noff[n];
+      float c[4] = {__uint_as_float((uint32_t)cr), __uint_as_float((uint32_t)(cr >> 32)),
+                    __uint_as_float((uint32_t)ci), __uint_as_float((uint32_t)(ci >> 32))};
+#pragma unroll
+      for (int lv = 0; lv < L; ++lv)
+#pragma unroll
+        for (int part = 0; part < 2; ++part) {
+          const __nv_bfloat162 v = __floats2bfloat162_rn(c[2 * part], c[2 * part + 1]);
+          *reinterpret_cast<__nv_bfloat162*>(p + (2 * lv + part) * g.c_plane) = v;
+          if (lv + 1 < L) {
+            c[2 * part] -= __low2float(v);
+            c[2 * part + 1] -= __high2float(v);
+          }
+        }
     }
   }
 }
@@ -1099,16 +1141,28 @@ extern "C" int ptn_cgemm_bf16x3(const ptn_cgemm_desc* d, void* stream) {
     if (smallk_pairs_ok(g, d->M)) {
       int64_t pb = (d->M / 2 + SMALLK_T - 1) / SMALLK_T;
       if (pb > 152 * 16) pb = 152 * 16;
+      // a plane's entries of a pair in 8-byte words
+      const bool dense = d->lda == d->K && d->a_plane % 4 == 0;
       switch (d->K) {
-#define PTN_SMALLK_PAIR(k)                                                                                     \
-  case k:                                                                                                       \
-    cgemm_smallk_pair_kernel<k><<<(unsigned)pb, SMALLK_T, 0, st>>>(A, d->lda, d->a_plane, B, d->ldb, g, d->levels); \
+#define PTN_SMALLK_PAIR_L(k, l)                                                                            \
+  if (dense) cgemm_smallk_pair_kernel<k, l, true><<<(unsigned)pb, SMALLK_T, 0, st>>>(A, d->lda, d->a_plane, \
+                                                                                     B, d->ldb, g);         \
+  else cgemm_smallk_pair_kernel<k, l, false><<<(unsigned)pb, SMALLK_T, 0, st>>>(A, d->lda, d->a_plane, B,   \
+                                                                                d->ldb, g);
+#define PTN_SMALLK_PAIR(k)            \
+  case k:                             \
+    if (d->levels == 3) {             \
+      PTN_SMALLK_PAIR_L(k, 3)         \
+    } else {                          \
+      PTN_SMALLK_PAIR_L(k, 2)         \
+    }                                 \
     return ptn_launch_status();
         PTN_SMALLK_PAIR(2)
         PTN_SMALLK_PAIR(4)
         PTN_SMALLK_PAIR(6)
         PTN_SMALLK_PAIR(10)
 #undef PTN_SMALLK_PAIR
+#undef PTN_SMALLK_PAIR_L
         default:
           break;
       }

@@ -108,3 +108,39 @@ def test_every_store_gives_the_same_entries(lib, M, N, K, L, whole):
                 piece = x.to(torch.bfloat16)
                 assert torch.equal(p[2 * lv + part], piece), (name, lv)
                 x = x - piece.float()
+
+
+@pytest.mark.parametrize("K", [2, 4, 6, 10])
+@pytest.mark.parametrize("N", [1, 50, 128])
+@pytest.mark.parametrize("M,pad", [(2, 0), (254, 0), (600, 3), (600, 6), (40000, 0)])
+@pytest.mark.parametrize("L", [2, 3])
+def test_row_pairs_of_short_products(lib, K, N, M, pad, L):
+    """Products with K <= 10 on the FP32 units: two rows an instruction and rows read in
+    words must give what one row a thread gives (the complex128 output's kernel)."""
+    g = torch.Generator(device="cuda").manual_seed(K + N)
+    lda = K + pad
+    rows, cols, size = _layout("pairs", M, N)
+    plane = -(-M * lda // 8) * 8
+    A = torch.randn((2 * L, plane), device="cuda", generator=g).to(torch.bfloat16)
+    B = torch.randn((3 * L, N, -(-K // 8) * 8), device="cuda", generator=g).to(torch.bfloat16)
+    B[0::3] = -B[2::3]
+    got = {}
+    for kind in (0, 1):
+        from pytreenet_gb300 import _lib
+        d = _lib.CgemmDesc()
+        cp = -(-size // 8) * 8
+        C = torch.zeros((size if kind == 0 else 2 * L * cp,), device="cuda",
+                        dtype=torch.complex128 if kind == 0 else torch.bfloat16)
+        st = torch.zeros(1, dtype=torch.int32, device="cuda")
+        d.A, d.lda, d.a_plane, d.M, d.K = A.data_ptr(), lda, plane, M, K
+        d.Bx, d.ldb, d.N, d.out_kind, d.levels = B.data_ptr(), B.shape[-1], N, kind, L
+        d.C, d.c_plane, d.status = C.data_ptr(), cp, st.data_ptr()
+        _modes(d.m_out, rows)
+        _modes(d.n_out, cols)
+        assert lib.ptn_cgemm_bf16x3(ctypes.byref(d), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        got[kind] = C if kind == 0 else C.view(2 * L, cp)[:, :size]
+    for part, x in ((0, got[0].real.float()), (1, got[0].imag.float())):
+        for lv in range(L):
+            piece = x.to(torch.bfloat16)
+            assert torch.equal(got[1][2 * lv + part], piece)
+            x = x - piece.float()
