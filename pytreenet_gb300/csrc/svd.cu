@@ -202,12 +202,14 @@ __global__ void __launch_bounds__(SVD_THREADS) zsvd_jacobi_kernel(SvdArgs a) {
 // whatever the active lanes) and the chain poll - dot - rotation - update - send
 // of a round. So the four sums of a pair are reduced together (six additions
 // instead of twenty), one warp forms the rotation, with two reciprocal square
-// roots: with d = |b|^2 - |a|^2, h = sqrt(d^2 + 4 |a^H b|^2), q = |d| + h,
+// roots, while another one decides on it: with d = |b|^2 - |a|^2,
+// h = sqrt(d^2 + 4 |a^H b|^2), q = |d| + h,
 //   cos = q / sqrt(2 h q),  sin e^{i phi} = sign(d) 2 (a^H b) / sqrt(2 h q),
-// the smaller root as above; and the update is 12 FMAs per row. The matrix is
-// scaled by a power of two so that the squares stay in range. Measured: 128 x
-// 128 5.2 ms (18.2 ms with the grid barrier per round), 256 x 256 16.0 (61.0), 384
-// x 384 43.7 (123; more pairs than SMs).
+// the smaller root as above; and the update is 12 FMAs per row, those of V after
+// A's columns have been sent. The matrix is scaled by a power of two so that the
+// squares stay in range. Measured: 128 x 128 4.2 ms (18.2 ms with the grid barrier
+// per round; 5.2 with one warp for the decision and V's FMAs among A's), 256 x 256
+// 14.0 (61.0), 384 x 384 38.5 (123; more pairs than SMs).
 constexpr int RING_WARPS = 4;                        // per role: rows of A, rows of V
 constexpr int RING_ROWS = 32 * RING_WARPS;
 constexpr int RING_THREADS = 2 * RING_ROWS;
@@ -218,6 +220,11 @@ struct RingArgs {
   SvdArgs a;
   ulonglong2* box;          // [parity 2][CTA][slot 2][m + n][component 2]
 };
+
+// x 2^k for a normal x whose exponent stays in range.
+__device__ __forceinline__ double exp_add(double x, int k) {
+  return __hiloint2double(__double2hiint(x) + (k << 20), __double2loint(x));
+}
 
 // Sum over the warp of four values; every lane of quarter q (8 lanes) gets
 // value q.
@@ -388,10 +395,10 @@ __global__ void __launch_bounds__(RING_THREADS) zsvd_ring_kernel(RingArgs g) {
       const int ci = p == 0 ? 0 : 1 + (p - 1 + r) % (np - 1), cj = 1 + (np - 2 - p + r) % (np - 1);
       const bool swap = ci > cj;                     // the lower column is the rotation's first
       const int q = done & 1;
-      // (a warp that must leave tells the others at the round's barrier)
-      if (!ring_read<R>(box(done, p, swap ? 1 : 0), box(done, p, swap ? 0 : 1), tid, rows, done + 1, a.ctrl, a.status, x,
-                        y))
-        s_fail = 1;
+      // a warp that must leave tells the others at the round's barrier, so all leave
+      // there: none is left waiting at a barrier of its own
+      const int leave = !ring_read<R>(box(done, p, swap ? 1 : 0), box(done, p, swap ? 0 : 1), tid, rows, done + 1, a.ctrl,
+                                      a.status, x, y);
       if (!vrole) {
         double al = 0.0, be = 0.0;
         double2 ga = make_double2(0.0, 0.0);
@@ -404,7 +411,7 @@ __global__ void __launch_bounds__(RING_THREADS) zsvd_ring_kernel(RingArgs g) {
         const double part = warp_sum4(al, be, ga.x, ga.y, lane);
         if ((lane & 7) == 0) red[q][warp][lane >> 3] = part;
         asm volatile("bar.sync 1, %0;" ::"n"(RING_ROWS) : "memory");
-        if (warp == 0) {
+        if (warp < 2) {
           double v = red[q][(lane >> 2) & 3][lane & 3];
           v += __shfl_xor_sync(0xffffffffu, v, 4);
           v += __shfl_xor_sync(0xffffffffu, v, 8);
@@ -413,31 +420,33 @@ __global__ void __launch_bounds__(RING_THREADS) zsvd_ring_kernel(RingArgs g) {
           ga.x = __shfl_sync(0xffffffffu, v, 2);
           ga.y = __shfl_sync(0xffffffffu, v, 3);
           const double g2 = fma(ga.x, ga.x, ga.y * ga.y);
-          const bool turn = al > zero2 && be > zero2 && g2 > tol2 * al * be;
-          double c = 1.0, sr = 0.0, si = 0.0;
-          if (turn) {
-            const double d = be - al, xx = fma(d, d, 4.0 * g2);
-            const double h = xx * rsqrt(xx), qq = fabs(d) + h, rr = rsqrt(2.0 * h * qq);
-            const double f = d >= 0.0 ? 2.0 * rr : -2.0 * rr;
-            c = qq * rr;
-            sr = f * ga.x;
-            si = f * ga.y;
-            ++count;
-          }
-          if (lane == 0) {
-            rot[q][0] = c;
-            rot[q][1] = sr;
-            rot[q][2] = si;
-            rot[q][3] = turn ? 1.0 : 0.0;
+          if (warp == 1) {
+            const bool turn = al > zero2 && be > zero2 && g2 > tol2 * al * be;
+            if (turn) ++count;
+            if (lane == 0) rot[q][3] = turn ? 1.0 : 0.0;
+          } else {
+            // (a pair that is not rotated has no use for these; factors of two on
+            // the exponents, where there is a rotation nothing is zero)
+            const double d = be - al, xx = fma(d, d, exp_add(g2, 2));
+            const double h = xx * rsqrt(xx), qq = fabs(d) + h, rr = rsqrt(exp_add(h, 1) * qq);
+            const double f = exp_add(d >= 0.0 ? rr : -rr, 1);
+            const double sr = f * ga.x, si = f * ga.y, c = qq * rr;
+            if (lane == 0) {
+              rot[q][0] = c;
+              rot[q][1] = sr;
+              rot[q][2] = si;
+            }
           }
         }
       }
-      __syncthreads();
-      if (s_fail) return;
+      if (__syncthreads_or(leave)) return;
       const double c = rot[q][0], sr = rot[q][1], si = rot[q][2];
       const bool turn = rot[q][3] != 0.0;
       ulonglong2* ox = box(done + 1, to_x, slot_x);
       ulonglong2* oy = box(done + 1, to_y, slot_y);
+      // V's rows wait until A's are on their way: their FMAs fill the FP64 pipe while
+      // the neighbours' columns travel
+      if (vrole) asm volatile("bar.sync 2, %0;" ::"n"(RING_THREADS) : "memory");
 #pragma unroll
       for (int u = 0; u < R; ++u) {
         const int t = tid + RING_ROWS * u;
@@ -454,8 +463,9 @@ __global__ void __launch_bounds__(RING_THREADS) zsvd_ring_kernel(RingArgs g) {
           st_mail(oy + 2 * t, swap ? x[u] : y[u], done + 2);
         }
       }
+      if (!vrole) asm volatile("bar.arrive 2, %0;" ::"n"(RING_THREADS) : "memory");
     }
-    if (threadIdx.x == 0 && count) atomicAdd(a.ctrl + 8 + (sweep % (CTRL_WORDS - 8)), count);
+    if (threadIdx.x == 32 && count) atomicAdd(a.ctrl + 8 + (sweep % (CTRL_WORDS - 8)), count);
     if (!grid_barrier(a.ctrl, a.status)) return;
     converged = *((volatile unsigned*)(a.ctrl + 8 + (sweep % (CTRL_WORDS - 8)))) == 0u;
   }
