@@ -70,7 +70,10 @@ constexpr int OUT_LD = 5;                         // pitch of an epilogue warp's
 constexpr int GROUP_COLS = 2 * TN;                // [Re | Im]
 constexpr int SPECIAL = INT_MAX;                  // exponent of a row with a NaN or an infinity
 constexpr int NO_ENTRY = INT_MIN;                 // no entry of the row seen that is not zero
-constexpr int MAX_SPLIT_STAGES = 256;             // K per split (the offset table of the conversion)
+// K per split: the conversion's offset table (12 bytes a k) and its row maxima stay
+// within the 48 KB of shared memory that a launch gets without asking for more.
+constexpr int MAX_SPLIT_STAGES = 248;
+static_assert(MAX_SPLIT_STAGES % CHUNK_STAGES == 0 && MAX_SPLIT_STAGES * KS * 12 + 128 * 4 <= 48 * 1024, "");
 constexpr int64_t A_BYTES_MAX = 1ll << 30;        // digits of A held at once; more rows go in turns
 // Complex multiply-adds from which this path is taken: its three launches cost
 // 25 to 28 us where the FP64 kernels take 16 us (1024 x 32 x 32, 1.0 M), 24 us
