@@ -79,6 +79,8 @@ constexpr int64_t A_BYTES_MAX = 1ll << 30;        // digits of A held at once; m
 // 25 to 28 us where the FP64 kernels take 16 us (1024 x 32 x 32, 1.0 M), 24 us
 // (512 x 64 x 64, 2.1 M), 87 us (640 x 128 x 128, 10 M).
 constexpr int64_t PTN_ZTC_MIN_MACS = 3ll << 20;
+constexpr int64_t MIN_OUTPUTS = 256;              // fewer stay with the FP64 kernels
+constexpr int64_t WORK_MAX = 8ll << 30;           // workspace a caller is asked for at most
 constexpr long long WAIT_CYCLES = 4000000000LL;   // ~2 s at 2 GHz
 
 struct Plan {
@@ -692,6 +694,11 @@ bool make_plan(int64_t M, int64_t N, int64_t K, Plan& p) {
   p.tiles_m = (p.M + TM - 1) / TM;
   p.tiles_n = (p.N + TN - 1) / TN;
   const int64_t tiles = p.tiles_m * p.tiles_n;
+  // Both sides are padded to a 128 x 32 tile, and converting those zeros costs like
+  // anything else: a few outputs over a long K stay with the FP64 kernels (16 x 16 over
+  // 65536 194 us there, 211 here, 8 x 8 over 131072 172 and 351, 2 x 3 over a million 1.3
+  // and 2.4 ms; 30 x 30 over 8000 125 us there, 61 here).
+  if (M * N <= MIN_OUTPUTS) return false;
   int64_t want = tiles >= 152 ? 1 : 152 / tiles;
   if (want > p.stages / CHUNK_STAGES) want = p.stages / CHUNK_STAGES;
   const int64_t least = (p.stages + MAX_SPLIT_STAGES - 1) / MAX_SPLIT_STAGES;
@@ -717,7 +724,7 @@ bool make_plan(int64_t M, int64_t N, int64_t K, Plan& p) {
   o += p.tiles_n * p.stages * B_STAGE;
   p.off_part = up(o, 256);
   p.bytes = p.off_part + (p.splits > 1 ? 16 * p.splits * p.chunk_tiles * TM * p.N : 0);
-  return true;
+  return p.bytes <= WORK_MAX;    // (a K of a million and more)
 }
 
 // Threads along K: one stage per thread when the rows alone fill the GPU (the
