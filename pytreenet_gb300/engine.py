@@ -13,8 +13,9 @@ Data layout in HBM
 * workspace slots: contraction intermediates and Krylov basis, grown on demand
   and shared by all plans (one stream, so no two plans run at once).
 
-A contraction step is ``ptn_zcontract``: tensordot semantics, but the legs are
-addressed through strides, so no tensor is ever transposed in memory.
+A contraction step is ``ptn_zcontract_ws``: tensordot semantics, but the legs are
+addressed through strides, so no tensor is ever transposed in memory. Large ones
+run on the tensor cores, in a workspace slot of their own.
 """
 from __future__ import annotations
 
@@ -1525,9 +1526,9 @@ class DeviceNetwork:
 
     # Jacobi runs on the q x q core when q is at most this, or when the kept
     # rank could exceed half of q; otherwise a subspace iteration reduces T to
-    # max_bond_dim + SUBSPACE_OVERSAMPLE columns first. Up to 64 columns the
-    # Jacobi sweeps run in one CTA (shared memory, CTA barriers); above, every
-    # round of a sweep is a grid-wide barrier (~4 ms for a 128 x 128 core). The
+    # max_bond_dim + SUBSPACE_OVERSAMPLE columns first. The
+    # Jacobi sweeps of up to 512 columns run as a ring of CTAs (4.2 ms for a
+    # 128 x 128 core); above, every round is a grid-wide barrier. The
     # subspace iteration costs two QRs and a host round trip per iteration, so
     # below SVD_DIRECT_MAX it is taken only for kept ranks up to
     # SUBSPACE_SMALL_L columns and cores at least four times wider (measured on
