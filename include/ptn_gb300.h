@@ -74,12 +74,16 @@ int ptn_zcontract(const ptn_contract_desc* d, void* stream);
 
 /* The same contraction with device scratch: contractions with enough
  * arithmetic run as exact integer digit products on the tensor cores (operands
- * rounded at 2^-56 of each row's largest entry, sums exact, one rounding to
- * double), whose error is not above the FP64 kernels'; the others, and calls
- * with null, misaligned (256 bytes) or too little scratch, run as
- * ptn_zcontract. ptn_zcontract_work_bytes: the scratch the call needs, 0 when
- * the FP64 kernels take it (host arithmetic on the descriptor's sizes). The
- * result does not vary between runs. Same counterparts as ptn_zcontract. */
+ * rounded at 2^-64 of each row's largest entry, sums exact, one rounding to
+ * double). Where that would lose more of an output than an FP64 sum does --
+ * its own terms, sum_k |a_mk| |b_kn|, lie below 2^-9 sqrt(max(K, 64) / 64) of the product
+ * of the row's and the column's largest entry -- the output is summed in FP64, so
+ * the error of every output is bounded by its own terms as in ptn_zcontract.
+ * The other contractions, and calls with null, misaligned (256 bytes) or too
+ * little scratch, run as ptn_zcontract. ptn_zcontract_work_bytes: the scratch the
+ * call may use, 0 when it uses none (host arithmetic on the descriptor's
+ * sizes). The result does not vary between runs; a wait on the
+ * device that runs out leaves NaN. Same counterparts as ptn_zcontract. */
 int64_t ptn_zcontract_work_bytes(const ptn_contract_desc* d);
 int ptn_zcontract_ws(const ptn_contract_desc* d, void* work, int64_t work_bytes, void* stream);
 
