@@ -355,13 +355,17 @@ int ptn_krylov_gs_step(const void* Q, int64_t ldq, int32_t nq, void* w, int64_t 
  * come to the host in one synchronisation and the reference's decisions are
  * taken there (happy breakdown, the stop beta0 beta |exp(z T) e_1|_m < tol, the
  * basis capacity). With j0 = 0 the batch begins with beta0 = |x| and row 0 =
- * x / beta0. Outputs: m (steps that count), done, and after done the column
- * beta0 exp(z T_m) e_1 in coef, which ptn_krylov_combine writes out as
- * out = sum_i coef_i Q_i. T (host, ldt x ldt complex128) keeps the projection
- * between batches: column j holds the coefficients of step j, its subdiagonal
- * |w|. Host memory that the device copies into is pinned. All other pointers
- * are device memory. beta0 = 0 returns done with m = 0. PTN_ERR_NONFINITE for a
- * vector that is not finite; a nonzero *status_host is left to the caller. */
+ * x / beta0. Outputs: m (steps that count), done, and the column
+ * beta0 exp(z T_m) e_1 in coef where `have` is set, which ptn_krylov_combine writes
+ * out as out = sum_i coef_i Q_i. The column is formed here only while that is little
+ * work (few vectors, |z T| small); past that `open` is the first step whose decision is
+ * left to the caller, who finds its norms in norms_host, and a caller that stops
+ * without `have` forms the column. T (host, ldt x ldt complex128) keeps the
+ * projection between batches: column j holds the coefficients of step j, its subdiagonal
+ * |w|; all columns of the batch up to the stop are written. Host memory that the device
+ * copies into is pinned. All other pointers are device memory. beta0 = 0 returns done
+ * with m = 0. PTN_ERR_NONFINITE for a vector that is not finite; a nonzero *status_host
+ * is left to the caller. */
 typedef struct {
   const ptn_exec_op* ops;
   int32_t nops, nptrs;
@@ -383,6 +387,7 @@ typedef struct {
   double z_re, z_im, tol;
   double beta0;             /* out with j0 = 0, in afterwards                   */
   int32_t m, done;          /* out                                              */
+  int32_t have, open;       /* out: coef is written; first undecided step or -1 */
 } ptn_krylov_desc;
 int ptn_krylov_batch(ptn_krylov_desc* d, void* stream);
 int ptn_krylov_combine(const void* Q, int64_t n, int32_t m, const void* coef_host, void* out, void* stream);

@@ -97,7 +97,8 @@ class KrylovDesc(ctypes.Structure):
                 ("coef", ctypes.c_void_p), ("n", ctypes.c_int64), ("ldt", ctypes.c_int64),
                 ("qcap", ctypes.c_int32), ("j0", ctypes.c_int32), ("batch", ctypes.c_int32),
                 ("tridiagonal", ctypes.c_int32), ("z_re", ctypes.c_double), ("z_im", ctypes.c_double),
-                ("tol", ctypes.c_double), ("beta0", ctypes.c_double), ("m", ctypes.c_int32), ("done", ctypes.c_int32)]
+                ("tol", ctypes.c_double), ("beta0", ctypes.c_double), ("m", ctypes.c_int32), ("done", ctypes.c_int32),
+                ("have", ctypes.c_int32), ("open", ctypes.c_int32)]
 
 
 OP_ZCONTRACT, OP_CGEMM, OP_TO_PLANES, OP_EXPAND_B, OP_ZCONTRACT_WS = 0, 1, 2, 3, 4

@@ -7,13 +7,12 @@
 // table and issues every launch from C++, so a host language pays one foreign
 // call per matvec instead of one per kernel. ptn_krylov_gs_step does the same
 // for the vector work of one Lanczos/Arnoldi step, and ptn_krylov_batch for a
-// whole batch of steps with the host's decisions, which took longer in the host
-// language than the GPU's work on vectors of a few thousand entries (an
-// eigendecomposition of the m x m projection per step).
+// whole batch of steps with the host's decisions where they are little work, which
+// took longer in the host language than the GPU's work on vectors of a few thousand
+// entries (an eigendecomposition of the m x m projection per step).
 #include <algorithm>
 #include <cmath>
 #include <complex>
-#include <vector>
 
 #include "ptn_common.cuh"
 
@@ -97,54 +96,66 @@ namespace {
 
 using cd = std::complex<double>;
 
-// exp(z H) e_1 for the Hermitian m x m projection H: the symmetrised T, or its
-// real tridiagonal part. Taylor series over steps with |z H|_1 <= 1 each; the
-// terms of a step fall below 1e-18 after about 20.
-void projected_column(const cd* T, int64_t ldt, int m, bool tridiagonal, cd z, std::vector<cd>& H, cd* col,
-                      std::vector<cd>& term, std::vector<cd>& next) {
-  H.assign((size_t)m * m, cd(0.0, 0.0));
+// exp(z H) e_1 for the Hermitian m x m projection H (the symmetrised T, or its real
+// tridiagonal part) where that is little work: a Taylor series over steps with
+// |z H|_1 <= 1 each, whose terms fall below 1e-18 after about 20. False, and nothing
+// written, for more than TAYLOR_WORK steps times m^2, where an eigendecomposition, which
+// does not depend on the norm, is the better one: the caller has it. (All columns of a
+// solve on a CPU: 25 vectors at |z H| = 10 1.9 ms of series and 1.2 of eigendecompositions,
+// 64 at 50 121 and 11 ms, 64 at 500 1.2 s and 11 ms; a site update of a time step has 5 to
+// 9 vectors at 1 and below.) Also for a norm that is not a number.
+constexpr int TAYLOR_MAX_M = 32;
+constexpr double TAYLOR_WORK = 1024.0;
+bool projected_column(const cd* T, int64_t ldt, int m, bool tridiagonal, cd z, cd* col) {
+  if (m > TAYLOR_MAX_M) return false;
+  cd H[TAYLOR_MAX_M * TAYLOR_MAX_M], term[TAYLOR_MAX_M], next[TAYLOR_MAX_M];
   for (int i = 0; i < m; ++i)
     for (int j = 0; j < m; ++j) {
       if (!tridiagonal)
-        H[(size_t)i * m + j] = 0.5 * (T[i * ldt + j] + std::conj(T[j * ldt + i]));
+        H[i * m + j] = 0.5 * (T[i * ldt + j] + std::conj(T[j * ldt + i]));
       else if (i == j)
-        H[(size_t)i * m + j] = T[i * ldt + i].real();
+        H[i * m + j] = T[i * ldt + i].real();
       else if (i == j + 1)
-        H[(size_t)i * m + j] = H[(size_t)j * m + i] = T[i * ldt + j].real();
+        H[i * m + j] = T[i * ldt + j].real();
+      else if (j == i + 1)
+        H[i * m + j] = T[j * ldt + i].real();
+      else
+        H[i * m + j] = cd(0.0, 0.0);
     }
   double norm = 0.0;
   for (int j = 0; j < m; ++j) {
     double c = 0.0;
-    for (int i = 0; i < m; ++i) c += std::abs(H[(size_t)i * m + j]);
-    norm = std::max(norm, c);
+    for (int i = 0; i < m; ++i) c += std::abs(H[i * m + j]);
+    if (!(c <= norm)) norm = c;
   }
-  const double steps_d = std::ceil(norm * std::abs(z));
-  const long steps = steps_d < 1.0 ? 1 : (long)std::min(steps_d, 1e6);
-  const cd zs = z / (double)steps;
+  double steps = std::ceil(norm * std::abs(z));
+  if (steps < 1.0) steps = 1.0;
+  if (!(steps * m * m <= TAYLOR_WORK)) return false;
+  const cd zs = z / steps;
   std::fill(col, col + m, cd(0.0, 0.0));
   col[0] = 1.0;
-  for (long s = 0; s < steps; ++s) {
-    term.assign(col, col + m);
+  for (int s = 0; s < (int)steps; ++s) {
+    std::copy(col, col + m, term);
     for (int k = 1; k < 200; ++k) {
       double size = 0.0, total = 0.0;
-      next.assign(m, cd(0.0, 0.0));
+      const cd f = zs / (double)k;
       for (int i = 0; i < m; ++i) {
         double re = 0.0, im = 0.0;
         for (int j = 0; j < m; ++j) {
-          const cd a = H[(size_t)i * m + j], b = term[j];
+          const cd a = H[i * m + j], b = term[j];
           re += a.real() * b.real() - a.imag() * b.imag();
           im += a.real() * b.imag() + a.imag() * b.real();
         }
-        const cd f = zs / (double)k;
         next[i] = cd(re * f.real() - im * f.imag(), re * f.imag() + im * f.real());
         col[i] += next[i];
         size = std::max(size, std::max(std::fabs(next[i].real()), std::fabs(next[i].imag())));
         total = std::max(total, std::max(std::fabs(col[i].real()), std::fabs(col[i].imag())));
       }
-      term.swap(next);
+      std::copy(next, next + m, term);
       if (!(size > 1e-18 * total)) break;
     }
   }
+  return true;
 }
 
 struct Coefficients {
@@ -199,7 +210,8 @@ extern "C" int ptn_krylov_batch(ptn_krylov_desc* d, void* stream) {
                         cudaSuccess) ||
       cudaStreamSynchronize(s) != cudaSuccess)
     return PTN_ERR_LAUNCH;
-  d->done = 0;
+  d->done = d->have = 0;
+  d->open = -1;
   d->m = d->j0;
   if (d->status && *d->status_host != 0) return PTN_OK;      // the caller reports it
   if (d->j0 == 0) d->beta0 = d->norms_host[0];
@@ -213,27 +225,30 @@ extern "C" int ptn_krylov_batch(ptn_krylov_desc* d, void* stream) {
   cd* coef = static_cast<cd*>(d->coef);
   const cd z(d->z_re, d->z_im);
   const double floor_abs = 2.220446049250313e-16 * (double)n;
-  std::vector<cd> H, a, b;
-  bool have = false;
   for (int j = d->j0; j < J && !d->done; ++j) {
     const cd* c = hh + (int64_t)j * (j + 1);
     const double w0 = d->norms_host[1 + 2 * j], beta = d->norms_host[2 + 2 * j];
     for (int i = 0; i <= j; ++i) T[i * d->ldt + j] = c[i] + c[j + 1 + i];
     T[(j + 1) * d->ldt + j] = beta;
+    if (d->open >= 0) continue;                      // the caller decides from there on
     d->m = j + 1;
-    have = false;
-    if (!std::isfinite(beta)) return PTN_ERR_NONFINITE;
+    d->have = 0;
+    if (!std::isfinite(beta) || std::isnan(w0)) return PTN_ERR_NONFINITE;
     if (beta <= std::max(floor_abs, 1e-12 * w0)) {
       d->done = 1;
     } else if (d->tol > 0.0) {
-      projected_column(T, d->ldt, d->m, d->tridiagonal != 0, z, H, coef, a, b);
-      have = true;
+      d->have = projected_column(T, d->ldt, d->m, d->tridiagonal != 0, z, coef);
+      if (!d->have) {
+        d->open = j;
+        continue;
+      }
       if (beta0 * beta * std::abs(coef[d->m - 1]) < d->tol) d->done = 1;
     }
     if (j + 1 >= d->qcap) d->done = 1;
   }
-  if (!have) projected_column(T, d->ldt, d->m, d->tridiagonal != 0, z, H, coef, a, b);
-  for (int i = 0; i < d->m; ++i) coef[i] *= beta0;
+  if (d->open < 0 && d->done && !d->have) d->have = projected_column(T, d->ldt, d->m, d->tridiagonal != 0, z, coef);
+  if (d->have)
+    for (int i = 0; i < d->m; ++i) coef[i] *= beta0;
   return PTN_OK;
 }
 

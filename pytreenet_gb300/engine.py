@@ -757,9 +757,12 @@ class KrylovSolver:
         if isinstance(plan, MixedPlan) and plan.prep and not plan.hold:
             plan.prepare()
         max_steps = n if max_krylov_dim is None else min(n, int(max_krylov_dim))
+        if max_steps < 1:
+            raise ValueError(f"max_krylov_dim = {max_krylov_dim}: at least one Krylov vector")
         spec = self._spec_depth.get(n, 4) if n <= self.SPECULATE_MAX_N else 1
         self._ensure_Q(x, n, min(max_steps + 1, max(spec + 1, 8)))
         T = np.zeros((min(max_steps, 64) + 1,) * 2, dtype=complex)
+        floor_abs = np.finfo(float).eps * max(n, 1)
         d = _lib.KrylovDesc()
         z = complex(exp_factor) * dt
         d.x, d.n, d.tridiagonal, d.tol = x.data_ptr(), n, int(tridiagonal), float(krylov_tol)
@@ -795,10 +798,27 @@ class KrylovSolver:
                 code = int(st_host[0])
                 st.zero_()
                 raise _lib.PtnError(code, "tensor-core contraction inside the Krylov exponential")
+            m, beta0, done = d.m, d.beta0, bool(d.done)
+            if d.open >= 0:
+                # steps whose column is more than a short series (``small_propagator``):
+                # the decisions of ``expm``
+                sc_all = sc[:1 + 2 * J].numpy()
+                for jj in range(d.open, J):
+                    w0, beta = float(sc_all[1 + 2 * jj]), float(sc_all[2 + 2 * jj])
+                    m = jj + 1
+                    if not np.isfinite(beta):
+                        raise _lib.PtnError(3, "Krylov exponential: non-finite vector")
+                    if beta <= max(floor_abs, 1e-12 * w0):
+                        done = True
+                    elif krylov_tol > 0.0:
+                        col = small_propagator(self._proj(T, m, tridiagonal), dt, exp_factor)
+                        done = beta0 * beta * abs(col[m - 1]) < krylov_tol
+                    if done or jj + 1 >= self._qcap:
+                        done = True
+                        break
             j = J
-            if d.done or j >= max_steps:
+            if done or j >= max_steps:
                 break
-        m, beta0 = d.m, d.beta0
         if beta0 == 0.0:
             if out.data_ptr() != x.data_ptr():
                 out.copy_(x)
@@ -811,6 +831,9 @@ class KrylovSolver:
         ran = getattr(apply, "ran", None)
         if ran is not None:
             ran(j)                       # how often the operator was applied
+        if not d.have or m != d.m:
+            coef = np.ascontiguousarray(beta0 * small_propagator(self._proj(T, m, tridiagonal), dt, exp_factor))
+            d.coef = coef.ctypes.data
         if basis is not None:
             Q = ws.bufs["kry_Q"][:m * n].view(m, n)
             basis.update(Q=Q.clone(), T=self._proj(T, m, tridiagonal).copy(), beta0=beta0, m=m)
