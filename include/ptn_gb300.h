@@ -98,6 +98,10 @@ int64_t ptn_zcontract_splits(int64_t tiles, int64_t K, int64_t* k_chunk);
  * matrix Q with leading dimension ldq (elements). partial buffers are
  * device scratch of at least ptn_krylov_partials(n) * (nq + 1) complex128. */
 int64_t ptn_krylov_partials(int64_t n);
+/* CTAs of the one-launch form of ptn_krylov_gs_step on a device of `sms` SMs, 0
+ * where the vector does not fit in their shared memory and each pass is a launch.
+ * Host-only arithmetic. No counterpart in the reference. */
+int64_t ptn_krylov_fused_ctas(int64_t n, int64_t sms);
 
 /* h[i] (+)= sum_x conj(Q[i, x]) w[x] for i < nq; h is device complex128[nq].
  * accumulate != 0 adds to h instead of overwriting. */

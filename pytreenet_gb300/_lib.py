@@ -112,6 +112,7 @@ SIGNATURES = {
     "ptn_zcontract_ws": (ctypes.c_int, [ctypes.POINTER(ContractDesc), _P, _I64, _P]),
     "ptn_zcontract_splits": (_I64, [_I64, _I64, ctypes.POINTER(ctypes.c_int64)]),
     "ptn_krylov_partials": (_I64, [_I64]),
+    "ptn_krylov_fused_ctas": (_I64, [_I64, _I64]),
     "ptn_zdot_multi": (ctypes.c_int, [_P, _I64, _I32, _P, _I64, _P, _I32, _P, _P]),
     "ptn_zaxpy_multi": (ctypes.c_int, [_P, _I64, _I32, _P, _P, _I64, _P]),
     "ptn_dznrm2": (ctypes.c_int, [_P, _I64, _P, _P, _P]),

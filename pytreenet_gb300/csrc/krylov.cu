@@ -423,40 +423,48 @@ __global__ void __launch_bounds__(FT) gs_fused_kernel(const double2* __restrict_
   }
 }
 
-// CTAs of the fused step: enough entries each that the exchange of G partial
-// sums does not outweigh the pass.
-static inline int64_t fused_ctas(int64_t n) {
-  const int64_t g = (n + 127) / 128;
-  return g < FUSED_MAX_CTAS ? g : FUSED_MAX_CTAS;
+// CTAs of the fused step on a device of `sms` SMs: enough entries each that the
+// exchange of G partial sums does not outweigh the pass, one to an SM (all of them
+// wait on one another, so all have to be resident).
+static inline int64_t fused_ctas(int64_t n, int64_t sms) {
+  const int64_t g = (n + 127) / 128, most = sms < FUSED_MAX_CTAS ? sms : FUSED_MAX_CTAS;
+  return g < most ? g : most;
 }
-static inline int64_t fused_per_cta(int64_t n) { return (n + fused_ctas(n) - 1) / fused_ctas(n); }
+
+// CTAs of the one-launch Gram-Schmidt step, 0 where w does not fit in their shared memory.
+extern "C" int64_t ptn_krylov_fused_ctas(int64_t n, int64_t sms) {
+  if (n < 1 || sms < 1) return 0;
+  const int64_t g = fused_ctas(n, sms), per = (n + g - 1) / g;
+  return per * (int64_t)sizeof(double2) <= FUSED_SMEM ? (n + per - 1) / per : 0;
+}
 
 template <int NQ>
 static int gs_step_nq(const double2* Q, int64_t ldq, double2* w, int64_t n, double2* h, double2* partial,
                       double* norms, double2* qnext, cudaStream_t s) {
   double* hd = reinterpret_cast<double*>(h);
-  const int64_t per = fused_per_cta(n);
-  // once per process, thread-safe
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      gs_fused_kernel<NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FUSED_SMEM);
-  if (attr == cudaSuccess && per * (int64_t)sizeof(double2) <= FUSED_SMEM) {
-    const int64_t g = (n + per - 1) / per;
+  static PtnSharedMemory shared_memory;
+  const int64_t g = ptn_krylov_fused_ctas(n, ptn_sm_count());
+  if (g > 0 && shared_memory((const void*)gs_fused_kernel<NQ>, FUSED_SMEM)) {
+    const int64_t most = fused_ctas(n, ptn_sm_count());
+    int64_t nn = n, pp = (n + most - 1) / most, ld = ldq;
     ulonglong2* mail = reinterpret_cast<ulonglong2*>(partial);
-    PTN_COUNT(1);
     if (g == 1) {                                    // nothing to exchange
-      gs_fused_kernel<NQ><<<1, FT, (size_t)per * sizeof(double2), s>>>(Q, ldq, w, n, per, hd, norms, qnext, mail);
+      PTN_COUNT(1);
+      gs_fused_kernel<NQ><<<1, FT, (size_t)pp * sizeof(double2), s>>>(Q, ldq, w, n, pp, hd, norms, qnext, mail);
       return ptn_launch_status();
     }
     if (cudaMemsetAsync(mail, 0, (size_t)(3 * (2 * NQ + 1) * g) * sizeof(ulonglong2), s) != cudaSuccess)
       return PTN_ERR_LAUNCH;
-    int64_t nn = n, pp = per, ld = ldq;
     void* args[] = {&Q, &ld, &w, &nn, &pp, &hd, &norms, &qnext, &mail};
-    if (cudaLaunchCooperativeKernel((const void*)gs_fused_kernel<NQ>, dim3((unsigned)g), dim3(FT), args,
-                                    (size_t)per * sizeof(double2), s) != cudaSuccess) {
-      cudaGetLastError();
-      return PTN_ERR_LAUNCH;
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void*)gs_fused_kernel<NQ>, dim3((unsigned)g), dim3(FT),
+                                                      args, (size_t)pp * sizeof(double2), s);
+    if (e == cudaSuccess) {
+      PTN_COUNT(1);
+      return ptn_launch_status();
     }
-    return ptn_launch_status();
+    cudaGetLastError();
+    // fewer SMs to this context than to the device: one launch per pass, below
+    if (e != cudaErrorCooperativeLaunchTooLarge) return PTN_ERR_LAUNCH;
   }
   const int nb = (int)nblocks_for(n);
   double* part = reinterpret_cast<double*>(partial);
@@ -512,7 +520,7 @@ int ptn_gs_step_passes(const void* Q, int64_t ldq, int32_t nq, void* w, int64_t 
 // per-CTA sums of the kernels above, and the mailboxes of the fused step
 extern "C" int64_t ptn_krylov_partials(int64_t n) {
   const int64_t per_pass = nblocks_for(n) * (MAXQ + 1) + 16;
-  const int64_t fused = 3 * (2 * FUSED_MAX_NQ + 1) * fused_ctas(n);
+  const int64_t fused = 3 * (2 * FUSED_MAX_NQ + 1) * fused_ctas(n, FUSED_MAX_CTAS);
   return per_pass > fused ? per_pass : fused;
 }
 

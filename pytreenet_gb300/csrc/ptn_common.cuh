@@ -56,3 +56,32 @@ __device__ __forceinline__ double2 warp_sum2(double2 v) {
   v.y = warp_sum(v.y);
   return v;
 }
+
+// A kernel's dynamic shared memory beyond 48 KB has to be allowed on every device that
+// runs it: once per device (0..63), thread-safe; a failure is tried again on the next call.
+struct PtnSharedMemory {
+  std::atomic<unsigned long long> allowed{0};
+  bool operator()(const void* kernel, size_t bytes) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return false;
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+    if (allowed.load(std::memory_order_acquire) & bit) return true;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    allowed.fetch_or(bit, std::memory_order_release);
+    return true;
+  }
+};
+
+// SMs of the current device, 0 on an error.
+static inline int ptn_sm_count() {
+  static std::atomic<int> known[64];
+  int dev = 0, v = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return 0;
+  if (dev < 64 && (v = known[dev].load(std::memory_order_relaxed)) > 0) return v;
+  if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  if (dev < 64) known[dev].store(v, std::memory_order_relaxed);
+  return v;
+}
