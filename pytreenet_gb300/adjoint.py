@@ -136,9 +136,13 @@ def _raw_contract(a, la, b, lb, lc, klabels, conj_a=False, conj_b=False, out=Non
         ent = (st, ops, wb)
         _DESCS[key] = ent
     st, ops, wb = ent
-    # scratch per call: contractions of several threads and streams may overlap
-    work = torch.empty(wb, dtype=torch.uint8, device=a.device) if wb else None
-    ptrs = (ctypes.c_void_p * 5)(None, work.data_ptr() if wb else None, a.data_ptr(), b.data_ptr(), out.data_ptr())
+    # scratch per call: contractions of several threads and streams may overlap (without
+    # memory for it they run on the FP64 kernels)
+    try:
+        work = torch.empty(wb, dtype=torch.uint8, device=a.device) if wb else None
+    except torch.OutOfMemoryError:
+        work = None
+    ptrs = (ctypes.c_void_p * 5)(None, work.data_ptr() if work is not None else None, a.data_ptr(), b.data_ptr(), out.data_ptr())
     check(_lib.load().ptn_exec_ops(ops, 1, ptrs, 5, E._stream_ptr()), "ptn_exec_ops")
     return out
 

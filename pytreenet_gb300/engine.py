@@ -70,19 +70,48 @@ class _BufferTable(dict):
 
 
 class Workspace:
-    """Named device scratch buffers that only grow."""
+    """Named device scratch buffers that only grow. The scratch of the digit products
+    (``SPARE``) is an exception: it goes when memory for anything else runs out, and
+    where there is none for it the FP64 kernels, which need none, take its steps."""
+
+    SPARE = "zc_work"
 
     def __init__(self, device):
         self.device = device
         self.gen = 0                    # bumped whenever a buffer is replaced
         self.bufs: dict[str, torch.Tensor] = _BufferTable(self)
+        self._declined = None           # size of SPARE that did not fit
+
+    def alloc(self, numel: int, dtype=CDT) -> torch.Tensor:
+        try:
+            return torch.empty(numel, dtype=dtype, device=self.device)
+        except torch.OutOfMemoryError:
+            if self.SPARE not in self.bufs:
+                raise
+            self.bufs.pop(self.SPARE)
+            self._declined = 1          # not taken again
+            return torch.empty(numel, dtype=dtype, device=self.device)
 
     def get(self, name: str, numel: int, dtype=CDT) -> torch.Tensor:
         b = self.bufs.get(name)
         if b is None or b.numel() < numel or b.dtype != dtype:
-            b = torch.empty(max(numel, 1), dtype=dtype, device=self.device)
+            b = self.alloc(max(numel, 1), dtype)
             self.bufs[name] = b
         return b[:numel]
+
+    def has_spare(self, numel: int) -> bool:
+        """Whether the slot ``SPARE`` holds ``numel`` entries, or can."""
+        b = self.bufs.get(self.SPARE)
+        if b is not None and b.numel() >= numel:
+            return True
+        if self._declined is not None and numel >= self._declined:
+            return False
+        try:
+            self.bufs[self.SPARE] = torch.empty(numel, dtype=CDT, device=self.device)
+        except torch.OutOfMemoryError:
+            self._declined = numel
+            return False
+        return True
 
     def ptr(self, name: str) -> int:
         return self.bufs[name].data_ptr()
@@ -265,8 +294,6 @@ class Plan:
         # scratch of the steps that run as digit products on the tensor cores
         # (one slot: the steps run one after the other)
         self.work = [contract_work_bytes(st.desc, ws.device) for st in steps]
-        if any(self.work):
-            self.ws_sizes["zc_work"] = (max(self.work) + 15) // 16
 
     def native_ops(self) -> "_NativeOps":
         """The plan's launch list, its workspace slots allocated."""
@@ -274,11 +301,14 @@ class Plan:
         if getattr(self, "_sized_at", None) != ws.gen:
             for name, n in self.ws_sizes.items():
                 ws.get(name, n)
+            # each step by itself: one that asks for too much does not take it from the others
+            spare = [bool(wb) and ws.has_spare((wb + 15) // 16) for wb in self.work]
             self._sized_at = ws.gen     # slots only grow: still large enough until one is replaced
-        if not hasattr(self, "_exec"):
-            self._exec = _NativeOps([(_lib.OP_ZCONTRACT_WS, st.desc, st.refs + (("ws", "zc_work"),)) if wb else
-                                     (_lib.OP_ZCONTRACT, st.desc, st.refs)
-                                     for st, wb in zip(self.steps, self.work)])
+            if getattr(self, "_spare", None) != spare:
+                self._spare = spare
+                self._exec = _NativeOps([(_lib.OP_ZCONTRACT_WS, st.desc, st.refs + (("ws", ws.SPARE),)) if tc else
+                                         (_lib.OP_ZCONTRACT, st.desc, st.refs)
+                                         for st, tc in zip(self.steps, spare)])
         return self._exec
 
     def run(self, x_ptr: int = 0, y_ptr: int = 0):
@@ -596,7 +626,7 @@ class KrylovSolver:
         if cur is not None and cur.numel() >= cap * n:
             self._qcap = cur.numel() // n
             return
-        Qn = torch.empty((cap * n,), dtype=CDT, device=x.device)
+        Qn = self.ws.alloc(cap * n)
         if cur is not None and self._qcap > 0:
             keep = min(cur.numel(), cap * n, self._qcap * n)
             Qn[:keep].copy_(cur[:keep])
