@@ -375,6 +375,15 @@ __global__ void __launch_bounds__(FT) gs_fused_kernel(const double2* __restrict_
   const int64_t x0 = blockIdx.x * per_cta;
   const int len = (int)(n - x0 < per_cta ? n - x0 : per_cta);
   const int64_t slot = (int64_t)NV * gridDim.x;
+  // norms[1] only grows, as the bits of a non-negative double: a CTA whose wait runs out
+  // leaves a NaN that no other one's result replaces. It starts from zero before this
+  // CTA's first sums are out; a CTA that gives up before the last exchange is missed there
+  // by all, so only later NaNs have to last.
+  unsigned long long* norm_bits = reinterpret_cast<unsigned long long*>(norms + 1);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    atomicExch(norm_bits, 0ull);
+    __threadfence();
+  }
   double2 hs[NQ], acc[NQ];
   double nacc = 0.0;
   auto clear = [&]() {
@@ -411,11 +420,14 @@ __global__ void __launch_bounds__(FT) gs_fused_kernel(const double2* __restrict_
     ok = gs_exchange<NQ, 2>(acc, nacc, red, tot, mail + 2 * slot);
   }
   if (!ok) {                                         // the caller sees a norm that is not a number
-    if (threadIdx.x == 0) norms[0] = norms[1] = NAN;
+    if (threadIdx.x == 0) {
+      norms[0] = NAN;
+      atomicMax(norm_bits, 0x7ff8000000000000ull);
+    }
     return;
   }
   const double nrm = sqrt(tot[2 * NQ]), inv = 1.0 / nrm;
-  if (blockIdx.x == 0 && threadIdx.x == 0) norms[1] = nrm;
+  if (blockIdx.x == 0 && threadIdx.x == 0) atomicMax(norm_bits, (unsigned long long)__double_as_longlong(nrm));
   for (int e = threadIdx.x; e < len; e += FT) {
     const double2 v = ws[e];
     w[x0 + e] = v;
