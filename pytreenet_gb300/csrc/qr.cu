@@ -231,19 +231,21 @@ __global__ void zero_cols_kernel(double2* __restrict__ A, const int64_t* __restr
 // What bounds a step on GB300 is the FP64 pipe and its latency: a warp
 // instruction holds a scheduler's FP64 unit for 64 cycles whatever the active
 // lanes. Hence four warps (one per scheduler) with several rows per thread, FMA
-// forms (4 per row and product), and sums of both parts of all of a CTA's columns
-// reduced together.
+// forms (4 per row of a dot product, 6 per row of an update), and sums of both parts of
+// all of a CTA's columns reduced together.
 constexpr int64_t QR_SMALL_M = 2048;
 constexpr int ST = 256;
 constexpr int HT = 128;                  // threads of the small-m kernels
 constexpr int HW = HT / 32;
 
-// c - x g
+// c - x g, rounded once at the size of c: an entry goes through k of these, and a
+// second rounding (two FMAs onto c, an instruction less per part) shows in the
+// factors' error, |Q R - A| / |A| of 512 x 256 1.04e-15 in place of 7.8e-16. Costs 9 %
+// there (1.75 and 1.91 ms).
 __device__ __forceinline__ double2 csub_mul(double2 c, double2 x, double2 g) {
-  c.x = fma(-x.x, g.x, c.x);
-  c.x = fma(x.y, g.y, c.x);
-  c.y = fma(-x.x, g.y, c.y);
-  c.y = fma(-x.y, g.x, c.y);
+  const double px = fma(x.x, g.x, -x.y * g.y), py = fma(x.x, g.y, x.y * g.x);
+  c.x -= px;
+  c.y -= py;
   return c;
 }
 
@@ -276,15 +278,15 @@ __device__ __forceinline__ Reflector make_reflector(double2 alpha, double xn2) {
   const double a2 = fma(alpha.x, alpha.x, alpha.y * alpha.y), n2 = a2 + xn2;
   if (!(n2 > 1e-290 && n2 < 1e290)) return make_reflector_far(alpha, n2);
   const bool pos = alpha.x >= 0.0;                   // beta = -sign(Re alpha) |(alpha, x)|
-  // one reciprocal square root for 1 / beta and, times n2, for beta itself with
-  // one correction; the reciprocal beside it does not wait for the correction
+  // one reciprocal square root for beta and 1 / beta, one correction for each
   const double rn = rsqrt(n2), r0 = n2 * rn;
   const double nrm = fma(fma(-r0, r0, n2), 0.5 * rn, r0);
-  const double rd = __drcp_rn(fma(2.0 * fabs(alpha.x), r0, a2 + n2));  // 1 / |alpha - beta|^2
+  const double ri = fma(fma(-nrm, rn, 1.0), rn, rn);
   h.beta = make_double2(pos ? -nrm : nrm, 0.0);
-  h.nb = pos ? rn : -rn;
+  h.nb = pos ? ri : -ri;
   h.tau = make_double2(fma(alpha.x, h.nb, 1.0), alpha.y * h.nb);  // (beta - alpha) / beta
-  h.s = make_double2((alpha.x - h.beta.x) * rd, -alpha.y * rd);
+  const double dx = alpha.x - h.beta.x, rd = __drcp_rn(fma(dx, dx, alpha.y * alpha.y));
+  h.s = make_double2(dx * rd, -alpha.y * rd);
   return h;
 }
 
@@ -488,8 +490,8 @@ inline unsigned grid1(int64_t n) {
 // barriers about 1.6, and 2.7 us a reflector when Q is formed. Two columns per CTA
 // rather than one: half as many readers of each x, one reduction for both.
 // Measured against flags with fences, 256 threads and scaled reflectors:
-// 512 x 256 3.28 -> 1.75 ms, 256 x 128 1.35 -> 0.64, 128 x 64 0.62 -> 0.28,
-// 16 x 8 0.086 -> 0.046, 2048 x 128 3.38 -> 2.66.
+// 512 x 256 3.28 -> 1.91 ms, 256 x 128 1.36 -> 0.68, 128 x 64 0.62 -> 0.30,
+// 16 x 8 0.083 -> 0.047, 2048 x 128 3.38 -> 3.02.
 constexpr long long HP_WAIT_CYCLES = 4000000000LL;   // ~2 s at 2 GHz
 constexpr unsigned long long HP_EMPTY = ~0ull;
 
