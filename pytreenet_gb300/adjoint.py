@@ -142,7 +142,8 @@ def _raw_contract(a, la, b, lb, lc, klabels, conj_a=False, conj_b=False, out=Non
         work = torch.empty(wb, dtype=torch.uint8, device=a.device) if wb else None
     except torch.OutOfMemoryError:
         work = None
-    ptrs = (ctypes.c_void_p * 5)(None, work.data_ptr() if work is not None else None, a.data_ptr(), b.data_ptr(), out.data_ptr())
+    ptrs = (ctypes.c_void_p * 5)(None, work.data_ptr() if work is not None else None, a.data_ptr(), b.data_ptr(),
+                                 out.data_ptr())
     check(_lib.load().ptn_exec_ops(ops, 1, ptrs, 5, E._stream_ptr()), "ptn_exec_ops")
     return out
 

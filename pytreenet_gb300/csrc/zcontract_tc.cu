@@ -614,7 +614,8 @@ __device__ __noinline__ void plain_listed(const GemmArgs& g, uint32_t item, int 
 #pragma unroll 1
   for (int t = lane / L; t - lane / L < count; t += 32 / L) {
     const int e = list[min(t, count - 1)];
-    const int64_t row_in_turn = (int64_t)tm * TM + (part & 3) * 32 + e / WC, n = (int64_t)tn * TN + (part >> 2) * WC + e % WC;
+    const int64_t row_in_turn = (int64_t)tm * TM + (part & 3) * 32 + e / WC;
+    const int64_t n = (int64_t)tn * TN + (part >> 2) * WC + e % WC;
     int64_t oa, om, ob, on;
     decode(g.c.m, g.m0 + row_in_turn, oa, om);
     decode(g.c.n, n, ob, on);
@@ -738,7 +739,9 @@ __device__ __forceinline__ int marked_in(const GemmArgs& g, uint32_t tile) {
   return c.x + c.y + c.z + c.w;
 }
 // Whether all of a tile is summed in FP64: the same for its copies, MMAs and epilogue.
-__device__ __forceinline__ bool skips_digits(const GemmArgs& g, uint32_t tile) { return marked_in(g, tile) > g.skip_tile; }
+__device__ __forceinline__ bool skips_digits(const GemmArgs& g, uint32_t tile) {
+  return marked_in(g, tile) > g.skip_tile;
+}
 
 // The guard's outputs, after the digits: the parts of all tiles that have some are dealt
 // out to the epilogue warps of all CTAs, one part of a tile to a CTA, so that the FP64
@@ -1307,14 +1310,11 @@ extern "C" int ptn_zcontract_ws(const ptn_contract_desc* d, void* work, int64_t 
   if (!work || (reinterpret_cast<uintptr_t>(work) & 255) || !make_plan(c.M, c.N, c.K, p) || work_bytes < p.bytes ||
       c.M * c.N * c.K < PTN_ZTC_PAYS)
     return ptn_zcontract(d, stream);
-  // once per process, thread-safe; a failure is returned on every call
-  static const bool attr =
-      cudaFuncSetAttribute(ptn_zgemm_digits_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) ==
-          cudaSuccess &&
-      cudaFuncSetAttribute(ptn_zgemm_digits_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) ==
-          cudaSuccess &&
-      cudaFuncSetAttribute(ptn_zguard_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GUARD_SMEM) == cudaSuccess;
-  if (!attr) return PTN_ERR_LAUNCH;
+  static PtnSharedMemory unit_memory, general_memory, guard_memory;
+  if (!unit_memory((const void*)ptn_zgemm_digits_kernel<true>, SMEM) ||
+      !general_memory((const void*)ptn_zgemm_digits_kernel<false>, SMEM) ||
+      !guard_memory((const void*)ptn_zguard_kernel, GUARD_SMEM))
+    return PTN_ERR_LAUNCH;
   if (p.swap) {
     const double2* t = c.A;
     c.A = c.B;
