@@ -491,7 +491,7 @@ def run_gb300(args, rank, world):
                 "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": (achieved / peak) if achieved else None,
                 "peak_source": peak_src + "; achieved counts algorithmic complex flops (8 per complex MAC); "
-                               "the digit products issue 34x as many tensor flops",
+                               "the digit products issue 36x as many tensor flops",
                 "traffic": None}
     roof.update({
         "algorithmic_flops_per_matvec": heff_flops / max(n_heff, 1),
